@@ -30,8 +30,10 @@
 #include <cub/device/device_scan.cuh>
 
 #include "../../include/xpbd_capi.h"
+#include "fused.cuh"
 #include "kernels.cuh"
 #include "render.cuh"
+#include "tiles.cuh"
 #include "xpbd_internal.h"
 
 namespace xpbd {
@@ -100,18 +102,13 @@ struct DBuf {
 	size_t bytes() const { return sizeof(T) * n; }
 };
 
-// Rows [0, n) in chunks of 256, each chunk sorted by row length (longest first): the
-// groups of a warp then run rows of similar length, and the chunk keeps them local
-static std::vector<int> length_order(int n, const std::vector<int>& off)
+// Rows in chunks of 256, each chunk sorted by list length (longest first): the groups of a
+// warp then run rows of similar length, and the chunk keeps them local
+static void length_order(std::vector<int>& rows, const std::vector<int>& off)
 {
-	std::vector<int> ord(n);
-	for (int r = 0; r < n; ++r) ord[r] = r;
-	for (int c0 = 0; c0 < n; c0 += 256) {
-		const int c1 = std::min(n, c0 + 256);
-		std::stable_sort(ord.begin() + c0, ord.begin() + c1,
+	for (size_t c0 = 0; c0 < rows.size(); c0 += 256)
+		std::stable_sort(rows.begin() + c0, rows.begin() + std::min(rows.size(), c0 + 256),
 			[&](int a, int b) { return off[a + 1] - off[a] > off[b + 1] - off[b]; });
-	}
-	return ord;
 }
 
 // Solver settings.  Like the reference's file-static settings (forward.cu:53-92,
@@ -141,7 +138,7 @@ struct Settings {
 	int kin_count = 0;
 	float kin_margin = 0.0f, kin_friction = 0.0f;
 	bool use_graph = true;
-	bool reorder = true;             // Morton order inside the engine (results unchanged)
+	bool reorder = true;             // curve order inside the engine (results unchanged)
 	int lanes_a = 0, lanes_b = 0;    // volume kernel lanes per cluster / node (0 = automatic)
 	dev::CmMaterial cm{ 1.0f, 0.1f, 0.1f, 0.1f, 1.0f, 1 };   // ChainMail material (forward.cu:66-71)
 	bool cm_frontier = true;         // ChainMail sweeps on work lists (false: every sweep dense)
@@ -177,7 +174,8 @@ public:
 
 	// ---- host topology (caller index space) and the internal order ----
 	std::vector<int> perm, inv;
-	std::vector<unsigned long long> lcode;   // Morton code in its component's box, per caller index
+	std::vector<unsigned long long> lcode;   // curve position in its component's box, per caller index
+	std::vector<int> comp_no;                // component number (by lowest caller index), per caller index
 	HostGraph graph;
 	HostClusters clusters;
 	HostEdgeColoring coloring;
@@ -267,10 +265,25 @@ public:
 	DBuf<int> off, nbr;
 	DBuf<float> ndist, nstiff, lam;
 	DBuf<int> vol_off, vol_idx, rev_off, rev_idx, mat_type, vol_gs_order;
-	DBuf<int> vol_idx_s, rev_idx_s;  // the same lists, rows sorted along the Morton curve
+	DBuf<int> vol_idx_s, rev_idx_s;  // the same lists, rows sorted along the curve
 	DBuf<int> gather_order;          // gather group -> node: nodes of similar reverse-list length side by side
 	DBuf<float> det_rest, v_rest, rest_len, sigma_rest, lam_vol;
 	DBuf<float4> rec;
+	// the volume gather's tiles (tiles.cuh): tiles, their rows, columns and masks; the rows
+	// that keep the list form
+	struct TilePlan {
+		DBuf<dev::VolTile> tiles;
+		DBuf<int> rows, lists;
+		DBuf<unsigned int> words;
+		int count = 0, list_count = 0;
+		long long words_used = 0;
+		void release()
+		{
+			tiles.release(); rows.release(); lists.release(); words.release();
+			count = list_count = 0;
+			words_used = 0;
+		}
+	} tiles;
 	DBuf<int2> gs_edge;
 	DBuf<float> gs_rest, gs_stiff, gs_lam;
 	DBuf<unsigned int> sc_keys;
@@ -389,7 +402,7 @@ public:
 	// the same substep as one cooperative launch, and the autotuner that times both forms
 	// on the first steps after a capture (they give identical results) and keeps the faster
 	// the step forms the autotuner chooses from, all with the same results: 0 the kernel
-	// sequence, 1 the fused launch, 2 and 3 the sequence with its distance and volume
+	// sequence, 1 the fused launch, 2 and 3 the sequence with its distance and solve
 	// kernels compiled for 6 and 8 resident blocks per SM
 	static constexpr int kForms = 4;
 	static constexpr int kFormOcc[kForms] = { 0, 0, 6, 8 };
@@ -468,7 +481,7 @@ public:
 		vol_off.release(); vol_idx.release(); rev_off.release(); rev_idx.release(); mat_type.release();
 		vol_idx_s.release(); rev_idx_s.release(); gather_order.release();
 		vol_gs_order.release(); det_rest.release(); v_rest.release(); rest_len.release(); sigma_rest.release();
-		lam_vol.release(); rec.release(); gs_edge.release(); gs_rest.release(); gs_stiff.release(); gs_lam.release();
+		lam_vol.release(); rec.release(); tiles.release(); gs_edge.release(); gs_rest.release(); gs_stiff.release(); gs_lam.release();
 		sc_keys.release(); sc_bucket.release(); sc_start.release(); sc_cursor.release(); sc_idx_sorted.release();
 		sc_contacts.release(); sc_counts.release(); sc_block_sums.release(); d_obj_id.release(); sc_dp.release();
 		nf_keys.release(); nf_bucket.release(); nf_start.release(); nf_p.release();
@@ -504,16 +517,42 @@ public:
 	}
 
 	// ------------------------------------------------------------------ build
-	// Internal order: device slot r holds the caller's Gaussian perm[r] (Morton order of the
+	// Internal order: device slot r holds the caller's Gaussian perm[r] (Hilbert order of the
 	// rest positions, so that graph, cluster and hash-cell neighbours sit close in memory);
 	// inv[perm[r]] = r.  Every topology is built in the caller's index space — the
 	// reference's construction order is index-dependent — and only then relabelled, with
 	// every list keeping its order, so the kernels see exactly the reference's sequences.
-	// 63-bit Morton code of each Gaussian's rest position within the box `lo`..`hi`
-	static unsigned long long morton_code(const float* p, const float* lo, const float* hi)
+	// Position of a rest position on the 63-bit Hilbert curve of the cube at `lo` with edge
+	// `ext` (Skilling's transposition form: Gray decode, then undo the excess work).  The
+	// curve has no jumps and the cube no preferred axis, so a run of consecutive Gaussians is
+	// a compact blob: 128 of them and their clusters' members span about 850 Gaussians, where
+	// the Morton curve of the box spans about 1,000 (100,000 Gaussians, 64-member clusters).
+	static unsigned long long curve_code(const float* p, const float* lo, float ext)
 	{
+		unsigned int X[3];
+		for (int a = 0; a < 3; ++a) {
+			float u = (p[a] - lo[a]) / ext;
+			if (!std::isfinite(u)) u = 0.0f;
+			X[a] = (unsigned int)(std::min(std::max(u, 0.0f), 1.0f) * 2097151.0f);
+		}
+		const unsigned int top = 1u << 20;
+		for (unsigned int q = top; q > 1; q >>= 1) {
+			const unsigned int low = q - 1;
+			for (int a = 0; a < 3; ++a) {
+				if (X[a] & q) X[0] ^= low;
+				else {
+					const unsigned int t = (X[0] ^ X[a]) & low;
+					X[0] ^= t;
+					X[a] ^= t;
+				}
+			}
+		}
+		X[1] ^= X[0];
+		X[2] ^= X[1];
+		unsigned int t = 0;
+		for (unsigned int q = top; q > 1; q >>= 1)
+			if (X[2] & q) t ^= q - 1;
 		auto spread = [](unsigned long long v) {
-			v &= 0x1fffffull;
 			v = (v | v << 32) & 0x1f00000000ffffull;
 			v = (v | v << 16) & 0x1f0000ff0000ffull;
 			v = (v | v << 8) & 0x100f00f00f00f00full;
@@ -521,20 +560,11 @@ public:
 			v = (v | v << 2) & 0x1249249249249249ull;
 			return v;
 		};
-		unsigned long long c = 0;
-		for (int a = 0; a < 3; ++a) {
-			const float ext = hi[a] > lo[a] ? hi[a] - lo[a] : 1.0f;
-			float u = (p[a] - lo[a]) / ext;
-			if (!std::isfinite(u)) u = 0.0f;
-			u = std::min(std::max(u, 0.0f), 1.0f);
-			c |= spread((unsigned long long)(u * 2097151.0f)) << a;
-		}
-		return c;
+		return spread(X[0] ^ t) << 2 | spread(X[1] ^ t) << 1 | spread(X[2] ^ t);
 	}
 
 	// Internal order: objects (graph components) one after another, in the order of their
-	// lowest caller index, each along the Morton curve of its own box; a single object
-	// gets the Morton order of the scene's box.  Objects that share space (a packed batch)
+	// lowest caller index, each along the curve of its own box.  Objects that share space (a packed batch)
 	// then keep their rows, and the cache lines they gather, to themselves.
 	void compute_order()
 	{
@@ -562,14 +592,20 @@ public:
 				if (std::isfinite(v)) { clo[3 * r + a] = std::min(clo[3 * r + a], v); chi[3 * r + a] = std::max(chi[3 * r + a], v); }
 			}
 		}
-		// Morton code within each component's own box: also orders the rows of the 4- and
+		// curve position within each component's own box: also orders the rows of the 4- and
 		// 8-lane volume lists the same way whatever the renumbering and whatever other
 		// objects share the scene
 		lcode.resize(n);
-		for (int i = 0; i < n; ++i) {
-			const int r = comp[i];
-			lcode[i] = morton_code(&in_pos[3 * i], &clo[3 * r], &chi[3 * r]);
-		}
+		parallel_for(n, [&](int i0, int i1) {
+			for (int i = i0; i < i1; ++i) {
+				const float* lo = &clo[3 * (size_t)comp[i]];
+				const float* hi = &chi[3 * (size_t)comp[i]];
+				const float ext = std::max(hi[0] - lo[0], std::max(hi[1] - lo[1], hi[2] - lo[2]));
+				lcode[i] = curve_code(&in_pos[3 * (size_t)i], lo, ext > 0.0f ? ext : 1.0f);
+			}
+		});
+		comp_no.resize(n);
+		for (int i = 0; i < n; ++i) comp_no[i] = rank[comp[i]];
 		for (int i = 0; i < n; ++i) perm[i] = i;
 		if (S.reorder && n > 1)
 			std::stable_sort(perm.begin(), perm.end(), [&](int a, int b) {
@@ -706,6 +742,117 @@ public:
 		return 0;
 	}
 
+	static int prepare_tile_kernels()
+	{
+		CK(cudaFuncSetAttribute(dev::k_tile_gather, cudaFuncAttributeMaxDynamicSharedMemorySize, dev::kVtSmem));
+		CK(cudaFuncSetAttribute(dev::k_substep_fused, cudaFuncAttributeMaxDynamicSharedMemorySize, dev::kVtSmem));
+		return 0;
+	}
+
+	// The gather's tiles of 128 rows.  Rows go along the curve, component by component, in
+	// equal tiles, so a tile depends on its component alone (an object's result is the same
+	// alone, packed with others or renumbered).  Rows without entries, rows of small
+	// components and of tiles that do not pay (k_tile_build) keep the list form, row by row.
+	int build_tiles(const std::vector<int>& off_h)
+	{
+		tiles.release();
+		std::vector<int> order(n), rank;
+		for (int r = 0; r < n; ++r) order[r] = r;
+		if (!S.reorder) {
+			std::stable_sort(order.begin(), order.end(), [&](int a, int b) {
+				if (comp_no[a] != comp_no[b]) return comp_no[a] < comp_no[b];
+				return lcode[a] < lcode[b];
+			});
+			rank.resize(n);
+			for (int r = 0; r < n; ++r) rank[order[r]] = r;
+		}
+		std::vector<dev::VolTile> list;
+		std::vector<int> rows, active, plain;
+		rows.reserve(n);
+		long long entries = 0;
+		for (int b = 0; b < n;) {
+			int e = b;
+			while (e < n && comp_no[perm[order[e]]] == comp_no[perm[order[b]]]) ++e;
+			active.clear();
+			for (int k = b; k < e; ++k) {
+				const int r = order[k], len = off_h[r + 1] - off_h[r];
+				if (e - b >= dev::kVtMinComponent && len > 0) {
+					active.push_back(r);
+					entries += len;
+				}
+				else
+					plain.push_back(r);
+			}
+			const long long count = (long long)active.size(), k = (count + dev::kVtRows - 1) / dev::kVtRows;
+			for (long long t = 0; t < k; ++t) {
+				const int a0 = (int)(count * t / k), a1 = (int)(count * (t + 1) / k), m = a1 - a0;
+				dev::VolTile v = {};
+				v.row0 = (int)rows.size();
+				v.nrows = m;
+				v.mid[0] = active[a0 + m / 8]; v.mid[1] = active[a0 + m / 2]; v.mid[2] = active[a0 + 7 * m / 8];
+				list.push_back(v);
+				rows.insert(rows.end(), active.begin() + a0, active.begin() + a1);
+			}
+			b = e;
+		}
+		const int candidates = (int)list.size();
+		CK(tiles.rows.alloc(n)); CK(tiles.lists.alloc(n));
+		tiles.list_count = 0;
+		if (!candidates) {
+			CK(tiles.tiles.alloc(1)); CK(tiles.words.alloc(32));
+		}
+		else if (run_tile_build(list, rows, entries, rank, order))
+			return -1;
+		// tiles that pay, then the rows of the others
+		std::vector<dev::VolTile> kept;
+		for (const auto& v : list)
+			if (v.cols) kept.push_back(v);
+			else plain.insert(plain.end(), rows.begin() + v.row0, rows.begin() + v.row0 + v.nrows);
+		std::sort(plain.begin(), plain.end());
+		length_order(plain, off_h);
+		tiles.count = (int)kept.size();
+		tiles.list_count = (int)plain.size();
+		if (tiles.count)
+			CK(cudaMemcpyAsync(tiles.tiles.p, kept.data(), sizeof(dev::VolTile) * kept.size(), cudaMemcpyHostToDevice, stream));
+		if (tiles.list_count)
+			CK(cudaMemcpyAsync(tiles.lists.p, plain.data(), sizeof(int) * plain.size(), cudaMemcpyHostToDevice, stream));
+		CK(cudaStreamSynchronize(stream));
+		return 0;
+	}
+
+	// columns and masks of the candidate tiles on the device; `list` comes back decided
+	int run_tile_build(std::vector<dev::VolTile>& list, const std::vector<int>& rows, long long entries,
+		const std::vector<int>& rank, const std::vector<int>& order)
+	{
+		DBuf<unsigned int> pool, bump;
+		DBuf<int> d_rank, d_order;
+		const size_t cap = (size_t)std::min<long long>(std::max(entries, 1ll), INT_MAX - 64);
+		CK(pool.alloc(cap)); CK(bump.alloc(1)); CK(tiles.tiles.alloc(list.size()));
+		CK(cudaMemsetAsync(bump.p, 0, sizeof(unsigned int), stream));
+		CK(cudaMemcpyAsync(tiles.tiles.p, list.data(), sizeof(dev::VolTile) * list.size(), cudaMemcpyHostToDevice, stream));
+		CK(cudaMemcpyAsync(tiles.rows.p, rows.data(), sizeof(int) * rows.size(), cudaMemcpyHostToDevice, stream));
+		if (!rank.empty()) {
+			CK(d_rank.alloc(n)); CK(d_order.alloc(n));
+			CK(cudaMemcpyAsync(d_rank.p, rank.data(), sizeof(int) * n, cudaMemcpyHostToDevice, stream));
+			CK(cudaMemcpyAsync(d_order.p, order.data(), sizeof(int) * n, cudaMemcpyHostToDevice, stream));
+		}
+		CK(cudaFuncSetAttribute(dev::k_tile_build, cudaFuncAttributeMaxDynamicSharedMemorySize, dev::kVtBuildSmem));
+		if (prepare_tile_kernels()) return -1;
+		dev::k_tile_build<<<(unsigned)list.size(), dev::kVtThreads, dev::kVtBuildSmem, stream>>>(n, tiles.tiles.p, tiles.rows.p,
+			rev_off.p, rev_idx.p, d_rank.p, d_order.p, pos_rest.p, pool.p, (unsigned int)cap, bump.p);
+		CK(cudaGetLastError());
+		unsigned int used = 0;
+		CK(cudaMemcpyAsync(&used, bump.p, sizeof(used), cudaMemcpyDeviceToHost, stream));
+		CK(cudaMemcpyAsync(list.data(), tiles.tiles.p, sizeof(dev::VolTile) * list.size(), cudaMemcpyDeviceToHost, stream));
+		CK(cudaStreamSynchronize(stream));
+		tiles.words_used = (long long)std::min<size_t>(used, cap);
+		CK(tiles.words.alloc(std::max<long long>(tiles.words_used, 32)));
+		CK(cudaMemcpyAsync(tiles.words.p, pool.p, sizeof(unsigned int) * (size_t)tiles.words_used, cudaMemcpyDeviceToDevice,
+			stream));
+		CK(cudaStreamSynchronize(stream));
+		return 0;
+	}
+
 	// rebuildVolumeClusters (forward.cu:9814-10403): host BFS/FPS, then rest covariance on the GPU
 	int rebuild_clusters()
 	{
@@ -725,7 +872,7 @@ public:
 		CK(cudaMemcpyAsync(rev_off.p, roff_i.data(), sizeof(int) * (n + 1), cudaMemcpyHostToDevice, stream));
 		CK(cudaMemcpyAsync(rev_idx.p, ridx_i.data(), sizeof(int) * ridx_i.size(), cudaMemcpyHostToDevice, stream));
 		{
-			// copies of both lists with every row sorted along the Morton curve of the component
+			// copies of both lists with every row sorted along the curve of the component
 			// (caller index breaking ties), for the 4- and 8-lane kernels: the lanes of a cluster
 			// read neighbouring Gaussians (fewer cache lines per warp load)
 			std::vector<unsigned long long> kcode(n);
@@ -750,7 +897,9 @@ public:
 			CK(cudaMemcpyAsync(vol_idx_s.p, vs.data(), sizeof(int) * vs.size(), cudaMemcpyHostToDevice, stream));
 			CK(cudaMemcpyAsync(rev_idx_s.p, rs.data(), sizeof(int) * rs.size(), cudaMemcpyHostToDevice, stream));
 			{
-				const std::vector<int> ord = length_order(n, roff_i);
+				std::vector<int> ord(n);
+				for (int r = 0; r < n; ++r) ord[r] = r;
+				length_order(ord, roff_i);
 				CK(gather_order.alloc(n));
 				CK(cudaMemcpyAsync(gather_order.p, ord.data(), sizeof(int) * n, cudaMemcpyHostToDevice, stream));
 				CK(cudaStreamSynchronize(stream));
@@ -758,6 +907,8 @@ public:
 			CK(cudaStreamSynchronize(stream));
 			build_mark(5);
 		}
+		if (build_tiles(roff_i)) return -1;
+		build_mark(5);
 		vol_gs_order.release();
 		std::vector<int> order_i(clusters.gs_order.size());
 		for (size_t t = 0; t < order_i.size(); ++t) order_i[t] = inv[clusters.gs_order[t]];
@@ -1180,13 +1331,19 @@ public:
 	template <typename K, typename... A>
 	void launch(int stage, dim3 grid, dim3 block, K kernel, A... args)
 	{
+		launch_shared(stage, grid, block, 0, kernel, args...);
+	}
+	// the same with `shared` bytes of dynamic shared memory per block
+	template <typename K, typename... A>
+	void launch_shared(int stage, dim3 grid, dim3 block, size_t shared, K kernel, A... args)
+	{
 		cudaEvent_t a = nullptr, b = nullptr;
 		if (profiling) {
 			a = next_event();
 			b = next_event();
 			cudaEventRecord(a, stream);
 		}
-		kernel<<<grid, block, 0, stream>>>(args...);
+		kernel<<<grid, block, shared, stream>>>(args...);
 		++launches;
 		if (profiling) {
 			cudaEventRecord(b, stream);
@@ -1291,6 +1448,19 @@ public:
 			(!S.use_volume || (vol_lanes() == 4 && S.lanes_a == 0 && gather_lanes() == 4)) && !S.use_angle && n > 0;
 	}
 
+	void enqueue_tile_gather(const float4* pin, float4* pout)
+	{
+		if (tiles.count)
+			launch_shared(ST_VOL_GATHER, dim3(tiles.count), dim3(dev::kVtThreads), dev::kVtSmem, dev::k_tile_gather, n,
+				(const StepParams*)d_params, pin, pout, (const dev::VolTile*)tiles.tiles.p, (const int*)tiles.rows.p,
+				(const unsigned int*)tiles.words.p, (const int*)rev_off.p, (const int*)rev_idx_s.p, (const float4*)rec.p,
+				(const float*)recz(), (const float*)rest_len.p);
+		if (tiles.list_count)
+			launch(ST_VOL_GATHER, blocks_for((long long)tiles.list_count * 4), dim3(kBlock), dev::k_volume_gather_group<4>, n,
+				(const StepParams*)d_params, pin, pout, (const int*)rev_off.p, (const int*)rev_idx_s.p, (const float4*)rec.p,
+				(const float*)recz(), (const float*)rest_len.p, (const int*)tiles.lists.p, tiles.list_count);
+	}
+
 	// one step as a single cooperative launch (results identical to enqueue_step's sequence)
 	int enqueue_step_fused()
 	{
@@ -1298,7 +1468,7 @@ public:
 			int dev_id = 0, sms = 0, per_sm = 0;
 			CK(cudaGetDevice(&dev_id));
 			CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev_id));
-			CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, dev::k_substep_fused, kBlock, 0));
+			CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, dev::k_substep_fused, kBlock, dev::kVtSmem));
 			if (per_sm <= 0) return fail("fused substep: no block of the kernel fits an SM");
 			fused_grid = sms * per_sm;
 		}
@@ -1315,6 +1485,8 @@ public:
 		A.off = off.p; A.nbr = nbr.p; A.ndist = ndist.p; A.nstiff = nstiff.p; A.lam = lam.p;
 		A.vol_off = vol_off.p; A.vol_idx = vol_idx_s.p; A.mat_type = mat_type.p; A.rev_off = rev_off.p;
 		A.rev_idx = rev_idx_s.p; A.det_rest = det_rest.p; A.rest_len = rest_len.p; A.rec = rec.p; A.recz = recz();
+		A.tiles = tiles.tiles.p; A.tile_rows = tiles.rows.p; A.tile_words = tiles.words.p; A.tile_count = tiles.count;
+		A.list_rows = tiles.lists.p; A.list_count = tiles.list_count;
 		A.pos_rest = pos_rest.p; A.shape_rest = shape_rest.p; A.shape_q = shape_q.p; A.ctr = d_ctr;
 		A.obj_id = d_obj_id.p; A.ext_kin = S.kin_ext.empty() ? nullptr : d_kin_ext.p; A.ext_range = d_kin_range.p;
 		A.pos_out3 = pos_out3.p; A.perm = d_perm.p;
@@ -1322,6 +1494,7 @@ public:
 		cudaLaunchConfig_t cfg = {};
 		cfg.gridDim = dim3(grid);
 		cfg.blockDim = dim3(kBlock);
+		cfg.dynamicSmemBytes = dev::kVtSmem;
 		cfg.stream = stream;
 		cudaLaunchAttribute attr[1];
 		attr[0].id = cudaLaunchAttributeCooperative;
@@ -1435,15 +1608,16 @@ public:
 							(const int*)vol_idx.p, (const float*)det_rest.p, (const int*)mat_type.p, lam_vol.p, rec.p, recz(), rl);
 					if (lb == 32)
 						launch(ST_VOL_GATHER, blocks_for((long long)N * 32), B, dev::k_volume_gather_group<32>, N, dp, cpin,
-							pout, (const int*)rev_off.p, (const int*)rev_idx.p, (const float4*)rec.p, (const float*)recz(), (const float*)rest_len.p, (const int*)gather_order.p);
+							pout, (const int*)rev_off.p, (const int*)rev_idx.p, (const float4*)rec.p, (const float*)recz(), (const float*)rest_len.p, (const int*)gather_order.p, N);
 					else if (lb == 8)
 						launch(ST_VOL_GATHER, blocks_for((long long)N * 8), B, dev::k_volume_gather_group<8>, N, dp, cpin,
-							pout, (const int*)rev_off.p, (const int*)rev_idx_s.p, (const float4*)rec.p, (const float*)recz(), (const float*)rest_len.p, (const int*)gather_order.p);
+							pout, (const int*)rev_off.p, (const int*)rev_idx_s.p, (const float4*)rec.p, (const float*)recz(), (const float*)rest_len.p, (const int*)gather_order.p, N);
+					else if (lb == 4 && S.lanes_b == 0)
+						// automatic: tiles on the tensor cores, the other rows from their lists (4 lanes per node)
+						enqueue_tile_gather(cpin, pout);
 					else if (lb == 4)
-						launch(ST_VOL_GATHER, blocks_for((long long)N * 4), B,
-							occ == 8 ? dev::k_volume_gather_occ<4, 8> : occ == 6 ? dev::k_volume_gather_occ<4, 6>
-							: dev::k_volume_gather_group<4>, N, dp, cpin,
-							pout, (const int*)rev_off.p, (const int*)rev_idx_s.p, (const float4*)rec.p, (const float*)recz(), (const float*)rest_len.p, (const int*)gather_order.p);
+						launch(ST_VOL_GATHER, blocks_for((long long)N * 4), B, dev::k_volume_gather_group<4>, N, dp, cpin,
+							pout, (const int*)rev_off.p, (const int*)rev_idx_s.p, (const float4*)rec.p, (const float*)recz(), (const float*)rest_len.p, (const int*)gather_order.p, N);
 					else
 						launch(ST_VOL_GATHER, G, B, dev::k_volume_gather_thread, N, dp, cpin, pout, (const int*)rev_off.p,
 							(const int*)rev_idx.p, (const float4*)rec.p, (const float*)recz(), (const float*)rest_len.p);
@@ -1670,6 +1844,8 @@ public:
 	struct ArenaSeg {
 		int slot = -1, row0 = 0, rows = 0;
 		long long e0 = 0, ne = 0, m0 = 0, nm = 0, r0 = 0, nr = 0;
+		int t0 = 0, nt = 0, l0 = 0, nl = 0;      // tiles, rows in the list form, the tiles' words
+		long long w0 = 0, nw = 0;
 		bool live = false;
 		std::vector<int> inv;   // session caller index -> row within the segment
 	};
@@ -1685,6 +1861,7 @@ public:
 			return fail("xpbd_b200_arena_new: invalid capacity (each of rows, edges, members, reverse entries "
 				"1..2^31-1: the CSR offsets are 32-bit)");
 		if (ensure_stream()) return -1;
+		if (prepare_tile_kernels()) return -1;
 		arena = true;
 		rows_cap = (int)rows; e_cap = edges; m_cap = members; r_cap = rev;
 		const size_t R = (size_t)rows;
@@ -1695,6 +1872,9 @@ public:
 		CK(off.alloc(R + 1)); CK(vol_off.alloc(R + 1)); CK(rev_off.alloc(R + 1));
 		CK(nbr.alloc((size_t)edges)); CK(ndist.alloc((size_t)edges)); CK(nstiff.alloc((size_t)edges));
 		CK(lam.alloc((size_t)edges)); CK(vol_idx_s.alloc((size_t)members)); CK(rev_idx_s.alloc((size_t)rev));
+		// a tile's words never outnumber its list entries (k_tile_build); at most a tile per 64 rows
+		CK(tiles.tiles.alloc(R / 64 + 1)); CK(tiles.rows.alloc(R)); CK(tiles.lists.alloc(R));
+		CK(tiles.words.alloc((size_t)std::min<long long>(rev, INT_MAX - 64)));
 		CK(cudaMemsetAsync(off.p, 0, sizeof(int), stream));
 		CK(cudaMemsetAsync(vol_off.p, 0, sizeof(int), stream));
 		CK(cudaMemsetAsync(rev_off.p, 0, sizeof(int), stream));
@@ -1752,6 +1932,9 @@ public:
 		const int rows = src.n;
 		const long long ne = src.graph.off[rows], nm = src.clusters.vol_off[rows], nr = src.clusters.rev_off[rows];
 		auto fits = [&]() {
+			if ((size_t)tiles.count + src.tiles.count > tiles.tiles.n ||
+				(size_t)(tiles.words_used + src.tiles.words_used) > tiles.words.n)
+				return false;
 			return rows_used + (long long)rows <= rows_cap && e_used + ne <= e_cap && m_used + nm <= m_cap &&
 				r_used + nr <= r_cap;
 		};
@@ -1791,6 +1974,15 @@ public:
 			copy_shift(src.rev_off.p, rev_off.p + r0, rows + 1, (int)g.r0) ||
 			copy_shift(src.rev_idx_s.p, rev_idx_s.p + g.r0, nr, g.row0))
 			return -1;
+		g.t0 = tiles.count; g.nt = src.tiles.count; g.w0 = tiles.words_used; g.nw = src.tiles.words_used;
+		g.l0 = tiles.list_count; g.nl = src.tiles.list_count;
+		if (copy_shift(src.tiles.rows.p, tiles.rows.p + r0, rows, g.row0) ||
+			copy_shift(src.tiles.lists.p, tiles.lists.p + g.l0, g.nl, g.row0))
+			return -1;
+		if (g.nt)
+			dev::k_tile_copy<<<g.nt, kBlock, 0, stream>>>(src.tiles.tiles.p, tiles.tiles.p + g.t0, src.tiles.words.p,
+				tiles.words.p, g.row0, 0, (int)g.w0, g.row0);
+		CK(cudaGetLastError());
 		dev::k_fill_int<<<blocks_for(rows), kBlock, 0, stream>>>(rows, d_obj_id.p + r0, g.slot);
 		// the inverse masses a pin release restores: the session's own saved ones while it
 		// has pins, else its current ones
@@ -1807,6 +1999,7 @@ public:
 			col_prev[col_key(g.slot, c)] = K;
 		}
 		rows_used += rows; e_used += ne; m_used += nm; r_used += nr;
+		tiles.count += g.nt; tiles.list_count += g.nl; tiles.words_used += g.nw;
 		n = rows_used;
 		segs.push_back(std::move(g));
 		++generation;
@@ -1832,6 +2025,7 @@ public:
 		while (!segs.empty() && !segs.back().live) {
 			const ArenaSeg& b = segs.back();
 			rows_used = b.row0; e_used = b.e0; m_used = b.m0; r_used = b.r0;
+			tiles.count = b.t0; tiles.list_count = b.l0; tiles.words_used = b.w0;
 			segs.pop_back();
 		}
 		n = rows_used;
@@ -1844,14 +2038,18 @@ public:
 	int arena_compact()
 	{
 		if (sync()) return -1;
-		size_t stage_bytes = 0;
+		size_t stage_bytes = 0, stage_tiles = 0;
 		for (const auto& g : segs)
-			if (g.live)
+			if (g.live) {
 				stage_bytes = std::max(stage_bytes, std::max({ sizeof(float4) * (size_t)g.rows, sizeof(float) * 3 * (size_t)g.rows,
 					sizeof(int) * (size_t)(g.rows + 1), sizeof(int) * (size_t)g.ne, sizeof(int) * (size_t)g.nm,
-					sizeof(int) * (size_t)g.nr }));
+					sizeof(int) * (size_t)g.nr, sizeof(int) * (size_t)g.nw, sizeof(int) * (size_t)g.nl }));
+				stage_tiles = std::max<size_t>(stage_tiles, g.nt);
+			}
 		DBuf<unsigned char> stage;
+		DBuf<dev::VolTile> stage_t;
 		if (stage_bytes) CK(stage.alloc(stage_bytes));
+		if (stage_tiles) CK(stage_t.alloc(stage_tiles));
 		auto move = [&](void* base, size_t elem, long long from, long long to, long long count) -> int {
 			if (from == to || count <= 0) return 0;
 			unsigned char* b = static_cast<unsigned char*>(base);
@@ -1865,8 +2063,8 @@ public:
 			return copy_shift(reinterpret_cast<const int*>(stage.p), base + to, count, delta);
 		};
 		std::vector<ArenaSeg> kept;
-		int rows = 0;
-		long long e = 0, m = 0, r = 0;
+		int rows = 0, nt = 0, nl = 0;
+		long long e = 0, m = 0, r = 0, words = 0;
 		for (auto& g : segs) {
 			if (!g.live) continue;
 			const int dr = rows - g.row0;
@@ -1886,13 +2084,27 @@ public:
 					move_shift(vol_idx_s.p, g.m0, m, g.nm, dr) || move_shift(rev_off.p, a, b, k + 1, (int)drv) ||
 					move_shift(rev_idx_s.p, g.r0, r, g.nr, dr))
 					return -1;
+				if (move_shift(tiles.rows.p, a, b, k, dr) || move_shift(tiles.lists.p, g.l0, nl, g.nl, dr)) return -1;
+				if (g.nt) {
+					CK(cudaMemcpyAsync(stage.p, tiles.words.p + g.w0, sizeof(int) * (size_t)g.nw, cudaMemcpyDeviceToDevice,
+						stream));
+					CK(cudaMemcpyAsync(stage_t.p, tiles.tiles.p + g.t0, sizeof(dev::VolTile) * g.nt, cudaMemcpyDeviceToDevice,
+						stream));
+					dev::k_tile_copy<<<g.nt, kBlock, 0, stream>>>(stage_t.p, tiles.tiles.p + nt,
+						reinterpret_cast<const unsigned int*>(stage.p), tiles.words.p, dr, (int)g.w0, (int)words, dr);
+					CK(cudaGetLastError());
+				}
+				g.l0 = nl;
+				g.t0 = nt; g.w0 = words;
 				g.row0 = rows; g.e0 = e; g.m0 = m; g.r0 = r;
 			}
 			rows += g.rows; e += g.ne; m += g.nm; r += g.nr;
+			nt += g.nt; nl += g.nl; words += g.nw;
 			kept.push_back(std::move(g));
 		}
 		segs.swap(kept);
 		rows_used = rows; e_used = e; m_used = m; r_used = r;
+		tiles.count = nt; tiles.list_count = nl; tiles.words_used = words;
 		n = rows_used;
 		++generation;
 		return sync();
@@ -3040,6 +3252,8 @@ XPBD_API int xpbd_b200_debug_int(const char* name, int* out, long long cap)
 	if (s == "vol_gs_order") return copy_host(E.clusters.gs_order, (long long)E.clusters.gs_order.size(), out, cap);
 	if (s == "vol_gs_color_offset")
 		return copy_host(E.clusters.gs_color_off, (long long)E.clusters.gs_color_off.size(), out, cap);
+	if (s == "gather_tiles")   // the volume gather's tiles, and the rows that keep the list form
+		return copy_host(std::vector<int>{ E.tiles.count, E.tiles.list_count }, 2, out, cap);
 	if (s == "obj_id") return copy_host(E.obj_id, N, out, cap);
 	if (s == "mat_type") return dev_to_caller(E, E.mat_type.p, 1, out, cap);
 	if (s == "gs_edge" || s == "gs_color_offset") {

@@ -862,7 +862,7 @@ __global__ void __launch_bounds__(kSmemBlock) k_volume_solve_smem(int n, const S
 }
 
 // Kernel A in one pass over the members (S lanes per cluster, members L, L+S, ... of
-// the Morton-sorted list on lane L, two in flight per trip): each lane accumulates,
+// the curve-sorted list on lane L, two in flight per trip): each lane accumulates,
 // relative to the leader's position, the count, first and second moments of its
 // members and the same moments weighted by inverse mass.  The centred covariance
 //   Sigma = (1 / (m+1)) sum (q - c)(q - c)^T = sum d d^T / (m+1) - c' c'^T
@@ -1006,6 +1006,9 @@ __global__ void __launch_bounds__(kBlock) k_volume_solve_onepass(int n, const St
 	solve_onepass_lane<S, true>((long long)blockIdx.x * blockDim.x + threadIdx.x, n, P, pin,
 		voff, vidx, det_rest, mat_type, lam_vol, rec, recz, read_lam);
 }
+// The distance and volume solve kernels compiled for MINB resident blocks per SM (fewer
+// registers, more warps in flight for these latency-bound gathers): the same per-item code,
+// so the same results; the autotuner picks among the forms by timing.
 template <int S, int MINB>
 __global__ void __launch_bounds__(kBlock, MINB) k_volume_solve_occ(int n, const StepParams* __restrict__ P,
 	const float4* __restrict__ pin, const int* __restrict__ voff, const int* __restrict__ vidx,
@@ -1179,11 +1182,11 @@ __device__ __forceinline__ void gather_group_lane(long long gtid, int n, const S
 	const float3 o = gather_finish(pi, avg, __ldg(rest_len + idx), P->under_relax);
 	pout[idx] = make_float4(o.x, o.y, o.z, p4.w);
 }
-// node of gather group g: order[g] when an order is given (nodes of similar reverse-list
-// length side by side, so the groups of a warp run even trip counts)
-__device__ __forceinline__ int ordered_node(const int* __restrict__ order, int g, int n)
+// node of gather group g of `count`: order[g] when an order is given (nodes of similar
+// reverse-list length side by side, so the groups of a warp run even trip counts); n: none
+__device__ __forceinline__ int ordered_node(const int* __restrict__ order, int g, int count, int n)
 {
-	return (order && g < n) ? __ldg(order + g) : g;
+	return g >= count ? n : (order ? __ldg(order + g) : g);
 }
 // the 4-lane form is latency bound on its record loads: compiled for 6 resident blocks
 // per SM (42 registers) it keeps more loads in flight (11.73 -> 11.46 ms per frame at 1M)
@@ -1191,25 +1194,11 @@ template <int S>
 __global__ void __launch_bounds__(kBlock, S == 4 ? 6 : 1) k_volume_gather_group(int n, const StepParams* __restrict__ P,
 	const float4* __restrict__ pin, float4* __restrict__ pout, const int* __restrict__ roff,
 	const int* __restrict__ ridx, const float4* __restrict__ rec, const float* __restrict__ recz,
-	const float* __restrict__ rest_len, const int* __restrict__ order)
+	const float* __restrict__ rest_len, const int* __restrict__ order, int count)
 {
 	const long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-	gather_group_lane<S, true>((long long)ordered_node(order, (int)(g / S), n) * S + (g & (S - 1)), n, P, pin, pout,
-		roff, ridx, rec, recz, rest_len);
-}
-
-// The distance, volume solve and gather kernels compiled for MINB resident blocks per SM
-// (fewer registers, more warps in flight for these latency-bound gathers): the same
-// per-item code, so the same results; the autotuner picks among the forms by timing.
-template <int S, int MINB>
-__global__ void __launch_bounds__(kBlock, MINB) k_volume_gather_occ(int n, const StepParams* __restrict__ P,
-	const float4* __restrict__ pin, float4* __restrict__ pout, const int* __restrict__ roff,
-	const int* __restrict__ ridx, const float4* __restrict__ rec, const float* __restrict__ recz,
-	const float* __restrict__ rest_len, const int* __restrict__ order)
-{
-	const long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-	gather_group_lane<S, true>((long long)ordered_node(order, (int)(g / S), n) * S + (g & (S - 1)), n, P, pin, pout,
-		roff, ridx, rec, recz, rest_len);
+	gather_group_lane<S, true>((long long)ordered_node(order, (int)(g / S), count, n) * S + (g & (S - 1)), n, P, pin,
+		pout, roff, ridx, rec, recz, rest_len);
 }
 
 // Kernel B, one thread per node (forward.cu:9187-9243)
@@ -2436,7 +2425,7 @@ __device__ __forceinline__ int sc_build_one(int i, const StepParams* __restrict_
 }
 
 // Candidate lists, one thread per particle (thread i builds particle i's list; particles
-// are numbered along a Morton curve of their rest positions, so a warp's particles
+// are numbered along a Hilbert curve of their rest positions, so a warp's particles
 // share most of their 27 cells).
 __global__ void __launch_bounds__(kBlock) k_sc_build_sorted(int n, const StepParams* __restrict__ P,
 	const float4* __restrict__ X, const float4* __restrict__ Pp, const float4* __restrict__ rest,
@@ -3107,124 +3096,6 @@ __global__ void __launch_bounds__(kBlock) k_deformed_shapes(int n, const float4*
 	out_quat[4 * o + 2] = (float)(qyv / qn);
 	out_quat[4 * o + 3] = (float)(qzv / qn);
 	atomicAdd(&ctr->shapes_deformed, 1u);
-}
-
-// ===========================================================================
-// The whole substep in one cooperative launch: predict, then per iteration distance,
-// volume solve and gather, shape matching and the projections, then the velocity
-// commit, with a grid-wide barrier between phases.  Every phase runs the same
-// per-item code as its own kernel (the *_row / *_lane functions above, with plain
-// loads for the data the launch itself writes), so the result is that of the kernel
-// sequence bit for bit; what changes is one launch per substep instead of one per
-// phase.  Covers the default forms (Jacobi distance, 4-lane one-pass volume solve and
-// gather, shape matching, colliders, ground, press, contact shapes); self-collision,
-// object mode and the Gauss-Seidel forms keep the kernel sequence.
-// ===========================================================================
-struct SubstepArgs {
-	int n, iters, use_distance, use_volume, use_shape, shape_robust, project;
-	const StepParams* P;
-	float4 *pos_curr, *pos_next, *pos_tmp, *vel;
-	float* lam_vol;
-	const float4* cshape;
-	const float* crmax;
-	float* crg;
-	const int *off, *nbr;
-	const float *ndist, *nstiff;
-	float* lam;
-	const int *vol_off, *vol_idx, *mat_type, *rev_off, *rev_idx;
-	const float *det_rest, *rest_len;
-	float4* rec;
-	float* recz;
-	const float4 *pos_rest, *shape_rest;
-	float4* shape_q;
-	DevCounters* ctr;
-	const int* obj_id;
-	const KinCollider* ext_kin;
-	const int2* ext_range;
-	float* pos_out3;
-	const int* perm;
-};
-
-// Grid-wide barrier of the fused launch (all blocks are co-resident: the launch is
-// cooperative).  Thread 0 of each block publishes its block's writes, arrives, and the
-// last to arrive opens the next generation; the wait is bounded (about 2^24 polls of at
-// least 64 ns): if it runs out, bar_timeout is set and the launch runs to its end with
-// the host reporting the error, instead of hanging the GPU.
-__device__ __forceinline__ void grid_barrier(DevCounters* __restrict__ ctr)
-{
-	__syncthreads();
-	if (threadIdx.x == 0) {
-		volatile unsigned int* gen = &ctr->bar_gen;
-		const unsigned int g = *gen;
-		__threadfence();
-		if (atomicAdd(&ctr->bar_count, 1u) + 1u == gridDim.x) {
-			ctr->bar_count = 0u;
-			__threadfence();
-			atomicAdd(&ctr->bar_gen, 1u);
-		}
-		else {
-			unsigned int polls = 0;
-			while (*gen == g) {
-				if (++polls > (1u << 24)) { atomicExch(&ctr->bar_timeout, 1u); break; }
-				__nanosleep(64);
-			}
-		}
-		__threadfence();
-	}
-	__syncthreads();
-}
-
-__global__ void __launch_bounds__(kBlock, 2) k_substep_fused(SubstepArgs A)
-{
-	DevCounters* ctr = A.ctr;
-	const long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-	const long long nth = (long long)gridDim.x * blockDim.x;
-	const int lane = threadIdx.x & 31;
-	const long long wbase = tid - lane;   // lane-group phases: whole warps iterate together
-	const int n = A.n;
-	const StepParams* P = A.P;
-	for (long long i = tid; i < n; i += nth)
-		predict_row((int)i, n, P, A.pos_curr, A.pos_next, A.vel, A.use_volume ? A.lam_vol : nullptr, A.cshape, A.crg);
-	grid_barrier(ctr);
-	float4* pin = A.pos_next;
-	float4* pout = A.pos_tmp;
-	for (int it = 0; it < A.iters; ++it) {
-		const int first = (it == 0), last = (it == A.iters - 1);
-		if (A.use_distance) {
-			for (long long i = tid; i < n; i += nth)
-				distance_row<false>((int)i, n, P, pin, pout, A.off, A.nbr, A.ndist, A.nstiff, A.lam, first ? 0 : 1,
-					last ? 0 : 1);
-			grid_barrier(ctr);
-			float4* t = pin; pin = pout; pout = t;
-		}
-		if (A.use_volume) {
-			for (long long b = wbase; b < 4LL * n; b += nth)
-				solve_onepass_lane<4, false>(b + lane, n, P, pin, A.vol_off, A.vol_idx, A.det_rest, A.mat_type, A.lam_vol,
-					A.rec, A.recz, first ? 0 : 1);
-			grid_barrier(ctr);
-			for (long long b = wbase; b < 4LL * n; b += nth)
-				gather_group_lane<4, false>(b + lane, n, P, pin, pout, A.rev_off, A.rev_idx, A.rec, A.recz, A.rest_len);
-			grid_barrier(ctr);
-			float4* t = pin; pin = pout; pout = t;
-		}
-		if (A.use_shape) {
-			for (long long i = tid; i < n; i += nth) {
-				if (A.shape_robust)
-					shape_row<true, false>((int)i, n, P, pin, pout, A.pos_rest, A.off, A.nbr, A.shape_rest, A.shape_q);
-				else
-					shape_row<false, false>((int)i, n, P, pin, pout, A.pos_rest, A.off, A.nbr, A.shape_rest, A.shape_q);
-			}
-			grid_barrier(ctr);
-			float4* t = pin; pin = pout; pout = t;
-		}
-		if (A.project) {
-			for (long long i = tid; i < n; i += nth)
-				project_row((int)i, n, P, pin, A.pos_curr, nullptr, nullptr, A.ctr, last ? 1 : 0, A.obj_id, A.ext_kin,
-					A.ext_range, nullptr, nullptr, A.cshape, A.crmax, A.crg);
-			grid_barrier(ctr);
-		}
-	}
-	for (long long i = tid; i < n; i += nth) velocity_row((int)i, n, P, A.pos_curr, pin, A.vel, A.pos_out3, A.perm, A.crg);
 }
 
 // ===========================================================================

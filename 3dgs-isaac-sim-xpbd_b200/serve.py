@@ -33,8 +33,10 @@ from . import bridge, scenes
 BYTES_PER_GAUSSIAN = 3200   # a session engine of its own: state, graph, clusters, transposed clusters, blackboard
 # arena bytes per row (Gaussian): 7 float4 state arrays, caller-order positions, order,
 # object id, multiplier, rest volume terms, material, cluster record, saved inverse
-# mass, three CSR row starts; per directed edge 16 B, per member and reverse entry 4 B
-ARENA_ROW_BYTES = 212
+# mass, three CSR row starts (212 B), the volume gather's tile rows, list rows and tiles (10 B)
+# and tile words (at most the reverse entries' size); per directed edge 16 B, per member and
+# reverse entry 4 B
+ARENA_ROW_BYTES = 222 + 4 * 68
 ARENA_EDGES, ARENA_MEMBERS, ARENA_REV = 12, 66, 68      # capacity per row (8-NN graph, 64-member clusters)
 
 

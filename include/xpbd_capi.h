@@ -214,7 +214,7 @@ XPBD_API void xpbd_b200_set_graph(int enabled);
 /* Step forms, all with the same results bit for bit: the kernel sequence (form 0); the
  * substep as ONE cooperative launch with grid-wide barriers between its phases (form 1,
  * where the configuration allows it: no self-collision, object mode or Gauss-Seidel
- * forms); the sequence with its distance and volume kernels compiled for 6 or 8
+ * forms); the sequence with its distance and volume solve kernels compiled for 6 or 8
  * resident blocks per SM (forms 2, 3).  Mode 0 (default) runs form 0, 1 runs form 1,
  * 2 lets the autotuner time every form on the first steps after each capture and keep
  * the fastest.  xpbd_b200_tuning fills out[7]: form in use, decided, mean trial ms of
@@ -226,7 +226,7 @@ XPBD_API int xpbd_b200_tuning(float* out);
  * visiting order; 0 from the reference's own 27-cell scan of the start-position hash
  * (selfColBuildKernel).  The lists are identical either way. */
 XPBD_API void xpbd_b200_set_selfcol_near(int enabled);
-/* 1 (default): keep Gaussians in Morton order inside the engine (caller order at the
+/* 1 (default): keep Gaussians in Hilbert order inside the engine (caller order at the
  * ABI; results identical); 0: caller order.  Takes effect at the next upload. */
 XPBD_API void xpbd_b200_set_reorder(int enabled);
 /* Per-kernel CUDA-event timing of subsequent steps (launches then go kernel by kernel). */
