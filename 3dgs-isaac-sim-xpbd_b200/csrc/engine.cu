@@ -264,6 +264,7 @@ public:
 	DBuf<float> pos_out3;
 	DBuf<int> off, nbr;
 	DBuf<float> ndist, nstiff, lam;
+	DBuf<unsigned int> ecode;        // neighbour and row (modulo 32) of each directed edge
 	DBuf<int> vol_off, vol_idx, rev_off, rev_idx, mat_type, vol_gs_order;
 	DBuf<int> vol_idx_s, rev_idx_s;  // the same lists, rows sorted along the curve
 	DBuf<int> gather_order;          // gather group -> node: nodes of similar reverse-list length side by side
@@ -402,8 +403,8 @@ public:
 	// the same substep as one cooperative launch, and the autotuner that times both forms
 	// on the first steps after a capture (they give identical results) and keeps the faster
 	// the step forms the autotuner chooses from, all with the same results: 0 the kernel
-	// sequence, 1 the fused launch, 2 and 3 the sequence with its distance and solve
-	// kernels compiled for 6 and 8 resident blocks per SM
+	// sequence, 1 the fused launch, 2 and 3 the sequence with its volume solve
+	// compiled for 6 and 8 resident blocks per SM
 	static constexpr int kForms = 4;
 	static constexpr int kFormOcc[kForms] = { 0, 0, 6, 8 };
 	cudaGraphExec_t graph_form[kForms] = {};
@@ -477,7 +478,7 @@ public:
 		obj_params.release(); obj_disp.release(); obj_w.release(); obj_boxes.release(); push_partial.release();
 		push_T.release(); obj_count.release(); sc_active.release(); sc_cross.release(); sc_accum.release();
 		obj_shift_valid = false;
-		pos_out3.release(); off.release(); nbr.release(); ndist.release(); nstiff.release(); lam.release();
+		pos_out3.release(); off.release(); nbr.release(); ndist.release(); nstiff.release(); lam.release(); ecode.release();
 		vol_off.release(); vol_idx.release(); rev_off.release(); rev_idx.release(); mat_type.release();
 		vol_idx_s.release(); rev_idx_s.release(); gather_order.release();
 		vol_gs_order.release(); det_rest.release(); v_rest.release(); rest_len.release(); sigma_rest.release();
@@ -693,13 +694,15 @@ public:
 			std::vector<float> nd(std::max(m, 1)), ns(std::max(m, 1));
 			for (int e = 0; e < m; ++e) { nd[e] = graph.ndist[src[e]]; ns[e] = graph.nstiff[src[e]]; }
 			CK(off.alloc(n + 1)); CK(nbr.alloc(std::max(m, 1))); CK(ndist.alloc(std::max(m, 1)));
-			CK(nstiff.alloc(std::max(m, 1))); CK(lam.alloc(std::max(m, 1)));
+			CK(nstiff.alloc(std::max(m, 1))); CK(lam.alloc(std::max(m, 1))); CK(ecode.alloc(std::max(m, 1)));
 			CK(cudaMemcpyAsync(off.p, off_i.data(), sizeof(int) * (n + 1), cudaMemcpyHostToDevice, stream));
 			if (m > 0) {
 				CK(cudaMemcpyAsync(nbr.p, nbr_i.data(), sizeof(int) * m, cudaMemcpyHostToDevice, stream));
 				CK(cudaMemcpyAsync(ndist.p, nd.data(), sizeof(float) * m, cudaMemcpyHostToDevice, stream));
 				CK(cudaMemcpyAsync(nstiff.p, ns.data(), sizeof(float) * m, cudaMemcpyHostToDevice, stream));
 			}
+			dev::k_edge_codes<<<blocks_for(n), kBlock, 0, stream>>>(n, 0, off.p, nbr.p, ecode.p);
+			CK(cudaGetLastError());
 			CK(shape_rest.alloc(n)); CK(shape_q.alloc(n));
 			CK(cudaMemsetAsync(shape_q.p, 0, shape_q.bytes(), stream));   // zero = identity start
 			dev::k_shape_rest<<<blocks_for(n), kBlock, 0, stream>>>(n, pos_rest.p, off.p, nbr.p, shape_rest.p);
@@ -1514,7 +1517,7 @@ public:
 	}
 
 	// one step's kernel sequence (the body of runXPBDSimulation); occ = 6 or 8 launches the
-	// distance and default volume kernels compiled for that many blocks per SM
+	// default volume solve compiled for that many blocks per SM
 	int enqueue_step(int occ = 0)
 	{
 		const int N = n;
@@ -1554,10 +1557,15 @@ public:
 				}
 			}
 			else if (S.use_distance) {
-				auto k = occ == 8 ? dev::k_distance_occ<8> : occ == 6 ? dev::k_distance_occ<6> : dev::k_distance_jacobi;
-				launch(ST_DISTANCE, G, B, k, N, (const StepParams*)d_params, (const float4*)pin,
-					pout, (const int*)off.p, (const int*)nbr.p, (const float*)ndist.p, (const float*)nstiff.p, lam.p,
-					first ? 0 : 1, last ? 0 : 1);
+				if (N <= 1 << dev::kCodeBits)
+					launch(ST_DISTANCE, blocks_for(N, dev::kDistWarps * 32), dim3(dev::kDistWarps * 32), dev::k_distance_jacobi, N,
+						(const StepParams*)d_params, (const float4*)pin, pout, (const int*)off.p,
+						(const unsigned int*)ecode.p, (const float*)ndist.p, (const float*)nstiff.p, lam.p, first ? 0 : 1,
+						last ? 0 : 1);
+				else
+					launch(ST_DISTANCE, G, B, dev::k_distance_rows, N, (const StepParams*)d_params, (const float4*)pin, pout,
+						(const int*)off.p, (const int*)nbr.p, (const float*)ndist.p, (const float*)nstiff.p, lam.p,
+						first ? 0 : 1, last ? 0 : 1);
 				std::swap(pin, pout);
 			}
 			if (S.use_volume) {
@@ -1871,7 +1879,7 @@ public:
 		CK(mat_type.alloc(R)); CK(rec.alloc(3 * rec_rows())); CK(inv_mass_saved.alloc(R));
 		CK(off.alloc(R + 1)); CK(vol_off.alloc(R + 1)); CK(rev_off.alloc(R + 1));
 		CK(nbr.alloc((size_t)edges)); CK(ndist.alloc((size_t)edges)); CK(nstiff.alloc((size_t)edges));
-		CK(lam.alloc((size_t)edges)); CK(vol_idx_s.alloc((size_t)members)); CK(rev_idx_s.alloc((size_t)rev));
+		CK(lam.alloc((size_t)edges)); CK(ecode.alloc((size_t)edges)); CK(vol_idx_s.alloc((size_t)members)); CK(rev_idx_s.alloc((size_t)rev));
 		// a tile's words never outnumber its list entries (k_tile_build); at most a tile per 64 rows
 		CK(tiles.tiles.alloc(R / 64 + 1)); CK(tiles.rows.alloc(R)); CK(tiles.lists.alloc(R));
 		CK(tiles.words.alloc((size_t)std::min<long long>(rev, INT_MAX - 64)));
@@ -1983,6 +1991,7 @@ public:
 			dev::k_tile_copy<<<g.nt, kBlock, 0, stream>>>(src.tiles.tiles.p, tiles.tiles.p + g.t0, src.tiles.words.p,
 				tiles.words.p, g.row0, 0, (int)g.w0, g.row0);
 		CK(cudaGetLastError());
+		dev::k_edge_codes<<<blocks_for(rows), kBlock, 0, stream>>>(rows, g.row0, off.p, nbr.p, ecode.p);
 		dev::k_fill_int<<<blocks_for(rows), kBlock, 0, stream>>>(rows, d_obj_id.p + r0, g.slot);
 		// the inverse masses a pin release restores: the session's own saved ones while it
 		// has pins, else its current ones
@@ -2094,6 +2103,8 @@ public:
 						reinterpret_cast<const unsigned int*>(stage.p), tiles.words.p, dr, (int)g.w0, (int)words, dr);
 					CK(cudaGetLastError());
 				}
+				dev::k_edge_codes<<<blocks_for(g.rows), kBlock, 0, stream>>>(g.rows, rows, off.p, nbr.p, ecode.p);
+				CK(cudaGetLastError());
 				g.l0 = nl;
 				g.t0 = nt; g.w0 = words;
 				g.row0 = rows; g.e0 = e; g.m0 = m; g.r0 = r;
@@ -3112,7 +3123,7 @@ XPBD_API void xpbd_b200_set_selfcol_near(int enabled) { engine().S.sc_near = ena
 XPBD_API int xpbd_b200_tuning(float* out)
 {
 	// [0] form in use (0 kernel sequence, 1 fused launch, 2 / 3 the sequence with 6 / 8
-	// blocks per SM for distance and volume), [1] 1 once decided, [2] [3] mean trial-step
+	// blocks per SM for the volume solve), [1] 1 once decided, [2] [3] mean trial-step
 	// ms of forms 0 and 1, [4] launches per step of the form in use, [5] [6] of forms 2, 3
 	const Engine& E = *cur_engine();
 	if (!out) return fail("xpbd_b200_tuning: null output");

@@ -287,12 +287,72 @@ __global__ void __launch_bounds__(kBlock) k_predict(int n, const StepParams* __r
 }
 
 // ---------------------------------------------------------------------------
-// distance constraints, Jacobi (forward.cu:6484-6571).  One thread per Gaussian over
-// its CSR row; the multiplier of each directed edge is owned by that thread, so it is
-// updated in place (the reference ping-pongs two arrays; the value sequence per edge
-// is the same).  The first iteration of a step reads no multiplier (they start at 0)
-// and the last stores none (they are reset next step).
+// distance constraints, Jacobi (forward.cu:6484-6571).  The multiplier of each directed edge
+// belongs to its row, so it is updated in place (the reference ping-pongs two arrays; the
+// value sequence per edge is the same).  The first iteration of a step reads no multiplier
+// (they start at 0) and the last stores none (they are reset next step).
 // ---------------------------------------------------------------------------
+// Quotients by a number that seldom changes: num / den to correct rounding from the stored
+// reciprocal and one residual step (Markstein's division), den's reciprocal recomputed when
+// den changes.
+struct StoredQuotient {
+	float den, inv;
+	__device__ __forceinline__ StoredQuotient() : den(1.0f), inv(1.0f) {}
+	__device__ __forceinline__ float operator()(float num, float d)
+	{
+		if (d != den) { den = d; inv = __frcp_rn(d); }
+		const float q = __fmul_rn(num, inv);
+		return __fmaf_rn(__fmaf_rn(-q, d, num), inv, q);
+	}
+};
+// alpha / dt^2 of an edge's stiffness, recomputed when the stiffness changes
+struct EdgeCompliance {
+	float ss, gc, dt2, stiff, value;
+	__device__ __forceinline__ EdgeCompliance(const StepParams* __restrict__ P)
+		: ss(P->stiffness_scale), gc(P->dist_compliance), dt2(fmaxf(P->dt * P->dt, 1e-8f)), stiff(NAN), value(0.0f)
+	{
+	}
+	__device__ __forceinline__ float operator()(float s)
+	{
+		if (s != stiff) {
+			stiff = s;
+			value = gc / fmaxf(s * ss, 1e-6f) / dt2;
+		}
+		return value;
+	}
+};
+// One directed edge i -> j: updates its multiplier and gives w_i dl grad; false where the edge
+// does nothing.  Roundings are explicit, so that every kernel that inlines it agrees bit for
+// bit.  Length and direction come from one reciprocal square root; a residual step brings the
+// length, which the rest length is subtracted from, to correct rounding.
+__device__ __forceinline__ bool distance_edge(float3 pi, float wi, float4 q4, float ims, float alpha_tilde, float rest,
+	StoredQuotient& quotient, float& lambda, float3& corr)
+{
+	const float x = pi.x - q4.x, y = pi.y - q4.y, z = pi.z - q4.z;
+	const float d2 = __fmaf_rn(z, z, __fmaf_rn(y, y, __fmul_rn(x, x)));
+	const float inv = __frsqrt_rn(d2);
+	const float d0 = __fmul_rn(d2, inv);
+	const float d = __fmaf_rn(__fmaf_rn(-d0, d0, d2), __fmul_rn(0.5f, inv), d0);
+	const float denom = __fadd_rn(__fadd_rn(wi, __fmul_rn(q4.w, ims)), alpha_tilde);
+	// d2 below 1e-14 is a length below 1e-7 (and a NaN d from d2 = 0 or infinity)
+	if (d2 < 1e-14f || denom < 1e-8f) return false;
+	const float dl = quotient(__fmaf_rn(-alpha_tilde, lambda, __fsub_rn(rest, d)), denom);
+	lambda = __fadd_rn(lambda, dl);
+	const float s = __fmul_rn(__fmul_rn(wi, dl), inv);
+	corr = make_float3(__fmul_rn(x, s), __fmul_rn(y, s), __fmul_rn(z, s));
+	return true;
+}
+__device__ __forceinline__ float3 distance_move(float3 pi, float4 sum, float under_relax)
+{
+	const float s = __fmul_rn(1.0f / sum.w, under_relax);
+	return make_float3(__fmaf_rn(sum.x, s, pi.x), __fmaf_rn(sum.y, s, pi.y), __fmaf_rn(sum.z, s, pi.z));
+}
+__device__ __forceinline__ float4 add4(float4 a, float4 b)
+{
+	return make_float4(__fadd_rn(a.x, b.x), __fadd_rn(a.y, b.y), __fadd_rn(a.z, b.z), __fadd_rn(a.w, b.w));
+}
+
+// one row by one thread (the fused substep's form)
 template <bool NC>
 __device__ __forceinline__ void distance_row(int idx, int n, const StepParams* __restrict__ P,
 	const float4* __restrict__ pin, float4* __restrict__ pout, const int* __restrict__ off,
@@ -302,63 +362,27 @@ __device__ __forceinline__ void distance_row(int idx, int n, const StepParams* _
 	if (idx >= n) return;
 	const float4 p4 = ldv<NC>(pin, idx);
 	const float3 pi = f3(p4);
-	const float ims = P->inv_mass_scale, ss = P->stiffness_scale, gc = P->dist_compliance;
+	const float ims = P->inv_mass_scale;
 	const float wi = p4.w * ims;
-	float3 accum = make_float3(0.0f, 0.0f, 0.0f);
-	int valid = 0;
-	const float dt = P->dt;
-	const float dt2 = fmaxf(dt * dt, 1e-8f);
-	const int e0 = off[idx], e1 = off[idx + 1];
-	// one edge of the row: its neighbour's position and its own multiplier, rest length
-	// and stiffness already loaded
-	auto edge_step = [&](int edge, float4 q4, float lambda, float rest, float stiff_e) {
-		const float3 diff = sub3(pi, f3(q4));
-		const float d = len3(diff);
-		if (d < 1e-7f) return;
-		const float C = d - rest;
-		const float3 grad = mul3(diff, 1.0f / d);
-		const float wj = q4.w * ims;
-		const float stiff = fmaxf(stiff_e * ss, 1e-6f);
-		const float alpha = gc / stiff;
-		const float alpha_tilde = alpha / dt2;
-		const float denom = (wi + wj) + alpha_tilde;
-		if (denom < 1e-8f) return;
-		const float dl = (-C - alpha_tilde * lambda) / denom;
-		lambda += dl;
-		if (write_lam) lam[edge] = lambda;
-		if (wi > 0.0f) {
-			accum = add3(accum, mul3(grad, wi * dl));
-			valid++;
-		}
-	};
-	// two edges per trip: their loads are in flight together; edges are applied in row
-	// order, so the result is that of the one-at-a-time loop bit for bit
-	int edge = e0;
-	for (; edge + 1 < e1; edge += 2) {
-		const int j0 = __ldg(nbr + edge), j1 = __ldg(nbr + edge + 1);
-		const float l0 = read_lam ? lam[edge] : 0.0f, l1 = read_lam ? lam[edge + 1] : 0.0f;
-		const bool ok0 = j0 >= 0 && j0 < n, ok1 = j1 >= 0 && j1 < n;
-		float4 q0 = make_float4(0.0f, 0.0f, 0.0f, 0.0f), q1 = q0;
-		if (ok0) q0 = ldv<NC>(pin, j0);
-		if (ok1) q1 = ldv<NC>(pin, j1);
-		const float r0 = __ldg(ndist + edge), r1 = __ldg(ndist + edge + 1);
-		const float s0 = __ldg(nstiff + edge), s1 = __ldg(nstiff + edge + 1);
-		if (ok0) edge_step(edge, q0, l0, r0, s0);
-		if (ok1) edge_step(edge + 1, q1, l1, r1, s1);
+	EdgeCompliance alpha(P);
+	StoredQuotient quotient;
+	float4 sum = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+	for (int e = off[idx], e1 = off[idx + 1]; e < e1; ++e) {
+		const int j = __ldg(nbr + e);
+		if (j < 0 || j >= n) continue;
+		float lambda = read_lam ? lam[e] : 0.0f;
+		float3 c;
+		if (!distance_edge(pi, wi, ldv<NC>(pin, j), ims, alpha(__ldg(nstiff + e)), __ldg(ndist + e), quotient, lambda, c))
+			continue;
+		if (write_lam) lam[e] = lambda;
+		if (wi > 0.0f) sum = add4(sum, make_float4(c.x, c.y, c.z, 1.0f));
 	}
-	if (edge < e1) {
-		const int j = __ldg(nbr + edge);
-		const float lambda = read_lam ? lam[edge] : 0.0f;
-		if (j >= 0 && j < n) edge_step(edge, ldv<NC>(pin, j), lambda, __ldg(ndist + edge), __ldg(nstiff + edge));
-	}
-	float3 out = pi;
-	if (wi > 0.0f && valid > 0) {
-		const float3 avg = mul3(accum, 1.0f / float(valid));
-		out = add3(pi, mul3(avg, P->under_relax));
-	}
+	const float3 out = sum.w > 0.0f ? distance_move(pi, sum, P->under_relax) : pi;
 	pout[idx] = make_float4(out.x, out.y, out.z, p4.w);
 }
-__global__ void __launch_bounds__(kBlock) k_distance_jacobi(int n, const StepParams* __restrict__ P,
+
+// rows past what an edge code holds (k_distance_jacobi)
+__global__ void __launch_bounds__(kBlock) k_distance_rows(int n, const StepParams* __restrict__ P,
 	const float4* __restrict__ pin, float4* __restrict__ pout, const int* __restrict__ off,
 	const int* __restrict__ nbr, const float* __restrict__ ndist, const float* __restrict__ nstiff,
 	float* __restrict__ lam, int read_lam, int write_lam)
@@ -366,14 +390,80 @@ __global__ void __launch_bounds__(kBlock) k_distance_jacobi(int n, const StepPar
 	distance_row<true>(blockIdx.x * blockDim.x + threadIdx.x, n, P, pin, pout, off, nbr, ndist, nstiff, lam, read_lam,
 		write_lam);
 }
-template <int MINB>
-__global__ void __launch_bounds__(kBlock, MINB) k_distance_occ(int n, const StepParams* __restrict__ P,
+
+// A warp per 32 rows.  Their edges are one run of the CSR arrays: the lanes take them 32 at a
+// time (coalesced, every lane busy whatever the rows' degrees, the loads of five trips in
+// flight together), leave each correction in shared memory, and then every lane adds its own
+// row's in row order.  With a thread per row, loading its 8 to 18 edges two at a time, the
+// kernel was bound by the wavefronts of strided loads and, in small scenes, by the chain of
+// dependent ones.  ecode: an edge's neighbour, and its row modulo 32 in the top five bits.
+// Measured (us per launch): 1,000,000
+// Gaussians 84 -> 71, 200,000 28 -> 21, 20,000 13.6 -> 10.8, 250,000 of degree 14 52 -> 34.
+constexpr int kDistWarps = 4;        // warps per block
+constexpr int kDistTrips = 5;        // edges per lane in flight
+constexpr int kDistWindow = 320;     // edges per pass: two batches of trips (mean degree 9.3: one pass)
+constexpr int kCodeBits = 27;
+__global__ void __launch_bounds__(kDistWarps * 32) k_distance_jacobi(int n, const StepParams* __restrict__ P,
 	const float4* __restrict__ pin, float4* __restrict__ pout, const int* __restrict__ off,
-	const int* __restrict__ nbr, const float* __restrict__ ndist, const float* __restrict__ nstiff,
+	const unsigned int* __restrict__ ecode, const float* __restrict__ ndist, const float* __restrict__ nstiff,
 	float* __restrict__ lam, int read_lam, int write_lam)
 {
-	distance_row<true>(blockIdx.x * blockDim.x + threadIdx.x, n, P, pin, pout, off, nbr, ndist, nstiff, lam, read_lam,
-		write_lam);
+	__shared__ float4 s_row[kDistWarps][32];            // the rows' positions
+	__shared__ float4 s_corr[kDistWarps][kDistWindow];  // corrections; w = 1 where the edge counts
+	const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+	const int row0 = (blockIdx.x * kDistWarps + w) * 32;
+	if (row0 >= n) return;
+	const int row = row0 + lane;
+	const int e0 = off[min(row, n)], e1 = off[min(row + 1, n)];
+	float4 p4 = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+	if (row < n) p4 = ld4(pin, row);
+	s_row[w][lane] = p4;
+	const int begin = __shfl_sync(0xffffffffu, e0, 0), end = __shfl_sync(0xffffffffu, e1, 31);
+	__syncwarp();
+	const float ims = P->inv_mass_scale;
+	EdgeCompliance alpha(P);
+	StoredQuotient quotient;
+	float4 sum = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+	for (int w0 = begin; w0 < end; w0 += kDistWindow) {
+		const int w1 = min(w0 + kDistWindow, end);
+		for (int b = w0; b < w1; b += 32 * kDistTrips) {
+			unsigned int code[kDistTrips];
+			float rest[kDistTrips], stiff[kDistTrips], l[kDistTrips];
+			float4 q[kDistTrips];
+			const int at = b + lane;
+#pragma unroll
+			for (int t = 0; t < kDistTrips; ++t)
+				if (at + 32 * t < w1) {
+					code[t] = __ldg(ecode + at + 32 * t);
+					rest[t] = __ldg(ndist + at + 32 * t);
+					stiff[t] = __ldg(nstiff + at + 32 * t);
+					l[t] = read_lam ? lam[at + 32 * t] : 0.0f;
+				}
+#pragma unroll
+			for (int t = 0; t < kDistTrips; ++t)
+				if (at + 32 * t < w1) q[t] = ld4(pin, (int)(code[t] & ((1u << kCodeBits) - 1u)));
+#pragma unroll
+			for (int t = 0; t < kDistTrips; ++t)
+				if (at + 32 * t < w1) {
+					const float4 own = s_row[w][code[t] >> kCodeBits];
+					const float wi = own.w * ims;
+					float4 out = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+					float3 c;
+					if (distance_edge(f3(own), wi, q[t], ims, alpha(stiff[t]), rest[t], quotient, l[t], c)) {
+						if (write_lam) lam[at + 32 * t] = l[t];
+						if (wi > 0.0f) out = make_float4(c.x, c.y, c.z, 1.0f);
+					}
+					s_corr[w][at - w0 + 32 * t] = out;
+				}
+		}
+		__syncwarp();
+#pragma unroll 2
+		for (int e = max(e0, w0); e < min(e1, w1); ++e) sum = add4(sum, s_corr[w][e - w0]);
+		__syncwarp();
+	}
+	if (row >= n) return;
+	const float3 out = sum.w > 0.0f ? distance_move(f3(p4), sum, P->under_relax) : f3(p4);
+	pout[row] = make_float4(out.x, out.y, out.z, p4.w);
 }
 
 // distance Gauss-Seidel, one colour: thread per undirected edge, in place
@@ -1006,9 +1096,9 @@ __global__ void __launch_bounds__(kBlock) k_volume_solve_onepass(int n, const St
 	solve_onepass_lane<S, true>((long long)blockIdx.x * blockDim.x + threadIdx.x, n, P, pin,
 		voff, vidx, det_rest, mat_type, lam_vol, rec, recz, read_lam);
 }
-// The distance and volume solve kernels compiled for MINB resident blocks per SM (fewer
-// registers, more warps in flight for these latency-bound gathers): the same per-item code,
-// so the same results; the autotuner picks among the forms by timing.
+// The volume solve compiled for MINB resident blocks per SM (fewer registers, more warps in
+// flight for its latency-bound gathers): the same per-item code, so the same results; the
+// autotuner picks among the forms by timing.
 template <int S, int MINB>
 __global__ void __launch_bounds__(kBlock, MINB) k_volume_solve_occ(int n, const StepParams* __restrict__ P,
 	const float4* __restrict__ pin, const int* __restrict__ voff, const int* __restrict__ vidx,
@@ -2816,6 +2906,16 @@ __global__ void k_set_positions(int n, const float* __restrict__ pos3, const int
 	const float x = pos3[3 * o], y = pos3[3 * o + 1], z = pos3[3 * o + 2];
 	pos[i] = make_float4(x, y, z, pos[i].w);
 	pos_out3[3 * o] = x; pos_out3[3 * o + 1] = y; pos_out3[3 * o + 2] = z;
+}
+
+// neighbour and row modulo 32 of each edge (k_distance_jacobi), for rows [row0, row0 + n)
+__global__ void k_edge_codes(int n, int row0, const int* __restrict__ off, const int* __restrict__ nbr,
+	unsigned int* __restrict__ ecode)
+{
+	const int i = blockIdx.x * blockDim.x + threadIdx.x;
+	if (i >= n) return;
+	const unsigned int r = (unsigned int)((row0 + i) & 31) << kCodeBits;
+	for (int e = off[row0 + i]; e < off[row0 + i + 1]; ++e) ecode[e] = r | (unsigned int)nbr[e];
 }
 
 // serving arena: copy of an index array with every non-negative entry shifted by delta
