@@ -118,10 +118,11 @@ __global__ void __launch_bounds__(kBlock, 2) k_substep_fused(SubstepArgs A)
 		}
 		if (A.use_shape) {
 			for (long long i = tid; i < n; i += nth) {
+				auto at = [&](int e) { return __ldg(A.nbr + e); };
 				if (A.shape_robust)
-					shape_row<true, false>((int)i, n, P, pin, pout, A.pos_rest, A.off, A.nbr, A.shape_rest, A.shape_q);
+					shape_row<true, false>((int)i, n, P, pin, pout, A.pos_rest, A.off, at, A.shape_rest, A.shape_q);
 				else
-					shape_row<false, false>((int)i, n, P, pin, pout, A.pos_rest, A.off, A.nbr, A.shape_rest, A.shape_q);
+					shape_row<false, false>((int)i, n, P, pin, pout, A.pos_rest, A.off, at, A.shape_rest, A.shape_q);
 			}
 			grid_barrier(ctr);
 			float4* t = pin; pin = pout; pout = t;

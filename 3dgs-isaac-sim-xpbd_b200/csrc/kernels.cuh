@@ -1605,140 +1605,97 @@ __device__ __forceinline__ bool shape_rotation_double(const M3& A, M3& Rout)
 	return ok;
 }
 
-// shape_rotation_double with the Jacobi started from the eigenvector frame of this
-// Gaussian's previous call (warm, a unit quaternion; all zero = identity) and that
-// frame stored back.  The polar factor R = U V^T is unique for a non-singular A, so the
-// start changes only where the iteration stops, not what it converges to (the same
-// 1e-12 relative off-diagonal test); successive calls of one Gaussian see nearly the
-// same A, which leaves one or two rotations instead of a full cold run.
-__device__ __forceinline__ bool shape_rotation_double_warm(const M3& A, M3& Rout, float4& warm)
+// rotation matrix of a quaternion close to unit length (2 / |q|^2 from the series of 1 / (1 + e))
+template <typename T>
+__device__ __forceinline__ void quat_matrix(const T (&q)[4], T (&R)[3][3])
 {
-	double a[3][3];
-#pragma unroll
-	for (int r = 0; r < 3; ++r)
-#pragma unroll
-		for (int c = 0; c < 3; ++c) a[r][c] = (double)A.m[c][r];
-	double m[3][3];
-#pragma unroll
-	for (int r = 0; r < 3; ++r)
-#pragma unroll
-		for (int c = 0; c < 3; ++c) m[r][c] = a[0][r] * a[0][c] + a[1][r] * a[1][c] + a[2][r] * a[2][c];
-	double v[3][3] = { { 1.0, 0.0, 0.0 }, { 0.0, 1.0, 0.0 }, { 0.0, 0.0, 1.0 } };
+	const T e = q[0] * q[0] + q[1] * q[1] + q[2] * q[2] + q[3] * q[3] - (T)1;
+	const T s = (T)2 - (T)2 * e * ((T)1 - e);
+	const T x = s * q[1], y = s * q[2], z = s * q[3];
+	R[0][0] = (T)1 - (y * q[2] + z * q[3]); R[0][1] = x * q[2] - z * q[0]; R[0][2] = x * q[3] + y * q[0];
+	R[1][0] = x * q[2] + z * q[0]; R[1][1] = (T)1 - (x * q[1] + z * q[3]); R[1][2] = y * q[3] - x * q[0];
+	R[2][0] = x * q[3] - y * q[0]; R[2][1] = y * q[3] + x * q[0]; R[2][2] = (T)1 - (x * q[1] + y * q[2]);
+}
+// q (1, w / 2): the rotation followed by one of about |w| (a Cayley step)
+template <typename T>
+__device__ __forceinline__ void quat_turn(T (&q)[4], T x, T y, T z)
+{
+	const T h = (T)0.5, a = q[0], b = q[1], c = q[2], d = q[3];
+	q[0] = a - h * (b * x + c * y + d * z);
+	q[1] = b + h * (a * x + c * z - d * y);
+	q[2] = c + h * (a * y + d * x - b * z);
+	q[3] = d + h * (a * z + b * y - c * x);
+}
+
+// The rotation of shapeMatchRotationDouble (polar factor of A, the smallest axis turned where
+// it would reflect) is the R in SO(3) that maximises tr(R^T A).  Newton's iteration on the
+// rotation finds it from the Gaussian's previous one: with B = R^T A,
+//   (tr B I - (B + B^T) / 2) w = axial(B - B^T),   R <- R exp([w]),
+// which converges cubically (the third-order term vanishes where B is symmetric).  FP32 steps
+// take it to FP32 rounding; then the residual axial(B - B^T) is formed in FP64 and corrected
+// with the FP32 matrix until the correction is below 3e-7, which leaves an error of 1e-12 or
+// less, the Jacobi iteration's own stop.  One step of each where the FP64 Jacobi run takes
+// AtA, two conjugations, one or two rotations and U V^T: about 80 FP64 operations for 350.
+// The matrix is positive definite only around the maximum, so a step that finds it is not
+// well so (its smallest eigenvalue, the sum of the two smallest singular values, under a
+// thousandth of its trace), a large step or a slow convergence go to the Jacobi run from
+// scratch.  warm: the rotation, a quaternion (all zero: identity).
+__device__ __forceinline__ bool shape_rotation_newton(const M3& A, M3& Rout, float4& warm)
+{
+	float q[4] = { warm.x, warm.y, warm.z, warm.w };
 	{
-		double qw = warm.x, qx = warm.y, qy = warm.z, qz = warm.w;
-		const double qn = qw * qw + qx * qx + qy * qy + qz * qz;
-		if (qn > 0.5) {
-			const double inv = 1.0 / sqrt(qn);
-			qw *= inv; qx *= inv; qy *= inv; qz *= inv;
-			v[0][0] = 1.0 - 2.0 * (qy * qy + qz * qz); v[0][1] = 2.0 * (qx * qy - qw * qz);
-			v[0][2] = 2.0 * (qx * qz + qw * qy);
-			v[1][0] = 2.0 * (qx * qy + qw * qz); v[1][1] = 1.0 - 2.0 * (qx * qx + qz * qz);
-			v[1][2] = 2.0 * (qy * qz - qw * qx);
-			v[2][0] = 2.0 * (qx * qz - qw * qy); v[2][1] = 2.0 * (qy * qz + qw * qx);
-			v[2][2] = 1.0 - 2.0 * (qx * qx + qy * qy);
-			// m <- V^T m V
-			double t[3][3];
-#pragma unroll
-			for (int r = 0; r < 3; ++r)
-#pragma unroll
-				for (int c = 0; c < 3; ++c) t[r][c] = m[r][0] * v[0][c] + m[r][1] * v[1][c] + m[r][2] * v[2][c];
-#pragma unroll
-			for (int r = 0; r < 3; ++r)
-#pragma unroll
-				for (int c = 0; c < 3; ++c) m[r][c] = v[0][r] * t[0][c] + v[1][r] * t[1][c] + v[2][r] * t[2][c];
-		}
+		const float n2 = q[0] * q[0] + q[1] * q[1] + q[2] * q[2] + q[3] * q[3];
+		if (!(n2 > 0.5f && n2 < 2.0f)) { q[0] = 1.0f; q[1] = q[2] = q[3] = 0.0f; }
 	}
-	for (int iter = 0; iter < 50; ++iter) {
-		bool done = true;
-		int piv = 0;   // 0: (0,1), 1: (0,2), 2: (1,2)
-		double max_off = -1.0;
+	float C00, C01, C02, C11, C12, C22;   // inverse of the Newton matrix
+	float w2 = 1.0f;
+	for (int it = 0; it < 5; ++it) {
+		float R[3][3], B[3][3];
+		quat_matrix(q, R);
 #pragma unroll
-		for (int k = 0; k < 3; ++k) {
-			const int pk = (k == 2) ? 1 : 0, qk = (k == 0) ? 1 : 2;
-			const double off = fabs(m[pk][qk]);
-			// off > 1e-12 sqrt(|a_pp a_qq|) + 1e-300, compared in squares (no square root)
-			if (off > 1e-300 && off * off > 1e-24 * fabs(m[pk][pk] * m[qk][qk])) done = false;
-			if (off > max_off) { max_off = off; piv = k; }
-		}
-		if (done) break;
-		if (piv == 0) jacobi_rotate_d<0, 1>(m, v);
-		else if (piv == 1) jacobi_rotate_d<0, 2>(m, v);
-		else jacobi_rotate_d<1, 2>(m, v);
+		for (int i = 0; i < 3; ++i)
+#pragma unroll
+			for (int k = 0; k < 3; ++k) B[i][k] = R[0][i] * A.m[k][0] + R[1][i] * A.m[k][1] + R[2][i] * A.m[k][2];
+		const float H00 = B[1][1] + B[2][2], H11 = B[0][0] + B[2][2], H22 = B[0][0] + B[1][1];
+		const float H01 = -0.5f * (B[0][1] + B[1][0]), H02 = -0.5f * (B[0][2] + B[2][0]), H12 = -0.5f * (B[1][2] + B[2][1]);
+		C00 = H11 * H22 - H12 * H12; C01 = H02 * H12 - H01 * H22; C02 = H01 * H12 - H02 * H11;
+		C22 = H00 * H11 - H01 * H01;
+		const float det = H00 * C00 + H01 * C01 + H02 * C02, tr = H00 + H11 + H22;
+		// positive definite, and by 4 det > 1e-3 tr^3 its smallest eigenvalue above 1e-3 tr
+		if (!(H00 > 0.0f && C22 > 0.0f && 4.0f * det > 1e-3f * tr * tr * tr)) return false;
+		C11 = H00 * H22 - H02 * H02; C12 = H01 * H02 - H00 * H12;
+		const float inv = 1.0f / det;
+		C00 *= inv; C01 *= inv; C02 *= inv; C11 *= inv; C12 *= inv; C22 *= inv;
+		const float ax = B[2][1] - B[1][2], ay = B[0][2] - B[2][0], az = B[1][0] - B[0][1];
+		const float x = C00 * ax + C01 * ay + C02 * az, y = C01 * ax + C11 * ay + C12 * az,
+			z = C02 * ax + C12 * ay + C22 * az;
+		w2 = x * x + y * y + z * z;
+		if (!(w2 < 0.25f)) return false;
+		quat_turn(q, x, y, z);
+		const float s = 1.5f - 0.5f * (q[0] * q[0] + q[1] * q[1] + q[2] * q[2] + q[3] * q[3]);   // to unit length, |w| small
+#pragma unroll
+		for (int k = 0; k < 4; ++k) q[k] *= s;
+		if (w2 < 1e-5f) break;
 	}
-	{
-		// the converged frame (a proper rotation: products of rotations), as a unit
-		// quaternion for the next call (largest-component extraction).  Kept in FP32: it
-		// only seeds the next call's Jacobi (re-normalised in FP64 there), whose stop test
-		// decides the result
-		float f[3][3];
-#pragma unroll
-		for (int r = 0; r < 3; ++r)
-#pragma unroll
-			for (int c = 0; c < 3; ++c) f[r][c] = (float)v[r][c];
-		const float tr = f[0][0] + f[1][1] + f[2][2];
-		float qw, qx, qy, qz;
-		if (tr > 0.0f) {
-			const float s2 = 2.0f * sqrtf(1.0f + tr), r2 = 1.0f / s2;
-			qw = 0.25f * s2; qx = (f[2][1] - f[1][2]) * r2; qy = (f[0][2] - f[2][0]) * r2; qz = (f[1][0] - f[0][1]) * r2;
-		} else if (f[0][0] > f[1][1] && f[0][0] > f[2][2]) {
-			const float s2 = 2.0f * sqrtf(fmaxf(1.0f + f[0][0] - f[1][1] - f[2][2], 1e-30f)), r2 = 1.0f / s2;
-			qw = (f[2][1] - f[1][2]) * r2; qx = 0.25f * s2; qy = (f[0][1] + f[1][0]) * r2; qz = (f[0][2] + f[2][0]) * r2;
-		} else if (f[1][1] > f[2][2]) {
-			const float s2 = 2.0f * sqrtf(fmaxf(1.0f + f[1][1] - f[0][0] - f[2][2], 1e-30f)), r2 = 1.0f / s2;
-			qw = (f[0][2] - f[2][0]) * r2; qx = (f[0][1] + f[1][0]) * r2; qy = 0.25f * s2; qz = (f[1][2] + f[2][1]) * r2;
-		} else {
-			const float s2 = 2.0f * sqrtf(fmaxf(1.0f + f[2][2] - f[0][0] - f[1][1], 1e-30f)), r2 = 1.0f / s2;
-			qw = (f[1][0] - f[0][1]) * r2; qx = (f[0][2] + f[2][0]) * r2; qy = (f[1][2] + f[2][1]) * r2; qz = 0.25f * s2;
-		}
-		warm = isfinite(qw + qx + qy + qz) ? make_float4(qw, qx, qy, qz) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+	if (!(w2 < 1e-5f)) return false;
+	double d[4] = { q[0], q[1], q[2], q[3] }, R[3][3];
+	double m2 = 1.0;
+	for (int it = 0; it < 4; ++it) {
+		quat_matrix(d, R);
+		const double ax = (R[0][2] * A.m[1][0] + R[1][2] * A.m[1][1] + R[2][2] * A.m[1][2]) -
+			(R[0][1] * A.m[2][0] + R[1][1] * A.m[2][1] + R[2][1] * A.m[2][2]);
+		const double ay = (R[0][0] * A.m[2][0] + R[1][0] * A.m[2][1] + R[2][0] * A.m[2][2]) -
+			(R[0][2] * A.m[0][0] + R[1][2] * A.m[0][1] + R[2][2] * A.m[0][2]);
+		const double az = (R[0][1] * A.m[0][0] + R[1][1] * A.m[0][1] + R[2][1] * A.m[0][2]) -
+			(R[0][0] * A.m[1][0] + R[1][0] * A.m[1][1] + R[2][0] * A.m[1][2]);
+		const double x = C00 * ax + C01 * ay + C02 * az, y = C01 * ax + C11 * ay + C12 * az,
+			z = C02 * ax + C12 * ay + C22 * az;
+		m2 = x * x + y * y + z * z;
+		quat_turn(d, x, y, z);
+		if (m2 < 1e-13) break;
 	}
-	double ev[3] = { m[0][0], m[1][1], m[2][2] };
-#pragma unroll
-	for (int i = 0; i < 2; ++i)
-#pragma unroll
-		for (int j = i + 1; j < 3; ++j)
-			if (ev[i] > ev[j]) {
-				const double te = ev[i]; ev[i] = ev[j]; ev[j] = te;
-#pragma unroll
-				for (int rr = 0; rr < 3; ++rr) { const double tv = v[rr][i]; v[rr][i] = v[rr][j]; v[rr][j] = tv; }
-			}
-	// singular values and their inverses from one reciprocal square root each (in place
-	// of a square root and a division: equal to FP64 rounding)
-	double S[3], Si[3];
-#pragma unroll
-	for (int i = 0; i < 3; ++i) {
-		Si[i] = ev[i] > 0.0 ? rsqrt(ev[i]) : 0.0;
-		S[i] = ev[i] > 0.0 ? ev[i] * Si[i] : 0.0;
-	}
-	const double smax = (S[2] > 1e-300) ? S[2] : 1e-300;
-#pragma unroll
-	for (int i = 0; i < 3; ++i) Si[i] = (S[i] > 1e-12 * smax) ? Si[i] : 0.0;
-	double u[3][3];
-#pragma unroll
-	for (int r = 0; r < 3; ++r)
-#pragma unroll
-		for (int c = 0; c < 3; ++c) u[r][c] = (a[r][0] * v[0][c] + a[r][1] * v[1][c] + a[r][2] * v[2][c]) * Si[c];
-	if (S[0] < 0.08 * smax) {
-		const double cx = u[1][1] * u[2][2] - u[2][1] * u[1][2];
-		const double cy = u[2][1] * u[0][2] - u[0][1] * u[2][2];
-		const double cz = u[0][1] * u[1][2] - u[1][1] * u[0][2];
-		const double len = sqrt(cx * cx + cy * cy + cz * cz);
-		if (!(len > 1e-7)) return false;
-		u[0][0] = cx / len; u[1][0] = cy / len; u[2][0] = cz / len;
-	}
-	double R[3][3];
-	for (int pass = 0; pass < 2; ++pass) {
-#pragma unroll
-		for (int r = 0; r < 3; ++r)
-#pragma unroll
-			for (int c = 0; c < 3; ++c) R[r][c] = u[r][0] * v[c][0] + u[r][1] * v[c][1] + u[r][2] * v[c][2];
-		const double det = R[0][0] * (R[1][1] * R[2][2] - R[1][2] * R[2][1])
-			- R[0][1] * (R[1][0] * R[2][2] - R[1][2] * R[2][0])
-			+ R[0][2] * (R[1][0] * R[2][1] - R[1][1] * R[2][0]);
-		if (det >= 0.0 || pass == 1) break;
-#pragma unroll
-		for (int rr = 0; rr < 3; ++rr) u[rr][0] = -u[rr][0];
-	}
+	if (!(m2 < 1e-13)) return false;
+	quat_matrix(d, R);
 	bool ok = true;
 #pragma unroll
 	for (int r = 0; r < 3; ++r)
@@ -1747,7 +1704,27 @@ __device__ __forceinline__ bool shape_rotation_double_warm(const M3& A, M3& Rout
 			ok = ok && isfinite(R[r][c]);
 			Rout.m[c][r] = (float)R[r][c];
 		}
+	warm = make_float4((float)d[0], (float)d[1], (float)d[2], (float)d[3]);
 	return ok;
+}
+// the same from scratch by the Jacobi iteration, and the rotation's quaternion
+__device__ __noinline__ bool shape_rotation_cold(const M3& A, M3& Rout, float4& warm)
+{
+	warm = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+	if (!shape_rotation_double(A, Rout)) return false;
+	const float(*m)[3] = Rout.m;   // m[column][row]
+	const float tr = m[0][0] + m[1][1] + m[2][2];
+	// the largest component first, the others from the off-diagonal sums and differences
+	const float a = m[1][2] - m[2][1], b = m[2][0] - m[0][2], c = m[0][1] - m[1][0];
+	const float xy = m[1][0] + m[0][1], xz = m[2][0] + m[0][2], yz = m[2][1] + m[1][2];
+	if (tr > 0.0f) warm = make_float4(1.0f + tr, a, b, c);
+	else if (m[0][0] > m[1][1] && m[0][0] > m[2][2]) warm = make_float4(a, 1.0f + m[0][0] - m[1][1] - m[2][2], xy, xz);
+	else if (m[1][1] > m[2][2]) warm = make_float4(b, xy, 1.0f + m[1][1] - m[0][0] - m[2][2], yz);
+	else warm = make_float4(c, xz, yz, 1.0f + m[2][2] - m[0][0] - m[1][1]);
+	const float n2 = warm.x * warm.x + warm.y * warm.y + warm.z * warm.z + warm.w * warm.w;
+	const float s = n2 > 1e-20f && n2 < 1e20f ? rsqrtf(n2) : 0.0f;
+	warm = make_float4(warm.x * s, warm.y * s, warm.z * s, warm.w * s);
+	return true;
 }
 
 __device__ __noinline__ bool shape_rotation_float(const M3& A, M3& Rout)
@@ -1823,14 +1800,13 @@ __global__ void __launch_bounds__(kBlock) k_shape_rest(int n, const float4* __re
 }
 
 // Per-iteration shape matching: current centroid, A = sum (p - c)(q - c_rest)^T over
-// {i} + 1-ring, normalised, rotation by polar decomposition (FP64 Jacobi when ROBUST,
-// else float), goal projection.  The rest-only terms come from k_shape_rest.  Three
-// blocks per SM (80 registers, a few spilled) hide more of the FP64 Jacobi chain's
-// latency than two (measured 1.3 -> 1.05 ms per substep at 1M).
-template <bool ROBUST, bool NC>
+// {i} + 1-ring, normalised, rotation by polar decomposition (to FP64 rounding when ROBUST,
+// else float), goal projection.  The rest-only terms come from k_shape_rest.  at(e): the
+// neighbour of edge e.
+template <bool ROBUST, bool NC, class Neighbour>
 __device__ __forceinline__ void shape_row(int idx, int n, const StepParams* __restrict__ P,
 	const float4* __restrict__ pin, float4* __restrict__ pout, const float4* __restrict__ rest,
-	const int* __restrict__ off, const int* __restrict__ nbr, const float4* __restrict__ shape_rest,
+	const int* __restrict__ off, const Neighbour& at, const float4* __restrict__ shape_rest,
 	float4* __restrict__ shape_q)
 {
 	if (idx >= n) return;
@@ -1866,7 +1842,7 @@ __device__ __forceinline__ void shape_row(int idx, int n, const StepParams* __re
 	};
 	int e = e0;
 	for (; e + 1 < e1; e += 2) {
-		const int j0 = __ldg(nbr + e), j1 = __ldg(nbr + e + 1);
+		const int j0 = at(e), j1 = at(e + 1);
 		const bool ok0 = j0 >= 0 && j0 < n, ok1 = j1 >= 0 && j1 < n;
 		float4 q0 = make_float4(0.0f, 0.0f, 0.0f, 0.0f), q1 = q0, r0 = q0, r1 = q0;
 		if (ok0) { q0 = ldv<NC>(pin, j0); r0 = ld4(rest, j0); }
@@ -1875,7 +1851,7 @@ __device__ __forceinline__ void shape_row(int idx, int n, const StepParams* __re
 		if (ok1) add(q1, r1);
 	}
 	if (e < e1) {
-		const int j = __ldg(nbr + e);
+		const int j = at(e);
 		if (j >= 0 && j < n) add(ldv<NC>(pin, j), ld4(rest, j));
 	}
 	const float3 com_curr = mul3(sq, sr.w);
@@ -1890,15 +1866,16 @@ __device__ __forceinline__ void shape_row(int idx, int n, const StepParams* __re
 		for (int r = 0; r < 3; ++r) a_norm_sq += A.m[c][r] * A.m[c][r];
 	const float a_norm = sqrtf(a_norm_sq);
 	if (!isfinite(a_norm) || a_norm < 1e-8f) { pout[idx] = p4; return; }
+	const float a_inv = 1.0f / a_norm;
 #pragma unroll
 	for (int c = 0; c < 3; ++c)
 #pragma unroll
-		for (int r = 0; r < 3; ++r) A.m[c][r] /= a_norm;
+		for (int r = 0; r < 3; ++r) A.m[c][r] *= a_inv;
 	M3 R;
 	bool ok;
 	if (ROBUST) {
 		float4 q = shape_q[idx];
-		ok = shape_rotation_double_warm(A, R, q);
+		ok = shape_rotation_newton(A, R, q) || shape_rotation_cold(A, R, q);
 		shape_q[idx] = q;
 	}
 	else {
@@ -1918,15 +1895,31 @@ __device__ __forceinline__ void shape_row(int idx, int n, const StepParams* __re
 	const float3 o = add3(pi, mul3(sub3(goal, pi), scale));
 	pout[idx] = make_float4(o.x, o.y, o.z, p4.w);
 }
-// four resident blocks per SM (64 registers, some spills): more warps hide the FP64
-// chain's latency better than fewer spills (measured against three and five)
+// A thread per Gaussian; a warp's edges are one run of the CSR array, so it brings their
+// neighbours to shared memory in a few coalesced loads first (one step of the dependent chain
+// less per trip; a run longer than the buffer is read in place).  Measured (us per launch,
+// the warm-started FP64 Jacobi -> this): 1,000,000 Gaussians 140 -> 100, 200,000 42 -> 27,
+// 20,000 17 -> 12.7.  Three blocks per SM (80 registers): four spill, 98 and 32 us, five 110
+// and 36.
+constexpr int kShapeWindow = 448;
 template <bool ROBUST>
-__global__ void __launch_bounds__(kBlock, 4) k_shape_match(int n, const StepParams* __restrict__ P,
+__global__ void __launch_bounds__(kBlock, 3) k_shape_match(int n, const StepParams* __restrict__ P,
 	const float4* __restrict__ pin, float4* __restrict__ pout, const float4* __restrict__ rest,
 	const int* __restrict__ off, const int* __restrict__ nbr, const float4* __restrict__ shape_rest,
 	float4* __restrict__ shape_q)
 {
-	shape_row<ROBUST, true>(blockIdx.x * blockDim.x + threadIdx.x, n, P, pin, pout, rest, off, nbr, shape_rest, shape_q);
+	__shared__ int s_nbr[kBlock / 32][kShapeWindow];
+	const int lane = threadIdx.x & 31;
+	const int row0 = blockIdx.x * blockDim.x + (threadIdx.x & ~31);
+	if (row0 >= n) return;
+	int* window = s_nbr[threadIdx.x >> 5];
+	const int begin = __ldg(off + row0), end = __ldg(off + min(row0 + 32, n));
+	const bool held = end - begin <= kShapeWindow;
+	if (held)
+		for (int e = begin + lane; e < end; e += 32) window[e - begin] = __ldg(nbr + e);
+	__syncwarp();
+	auto at = [&](int e) { return held ? window[e - begin] : __ldg(nbr + e); };
+	shape_row<ROBUST, true>(row0 + lane, n, P, pin, pout, rest, off, at, shape_rest, shape_q);
 }
 
 // ---------------------------------------------------------------------------
