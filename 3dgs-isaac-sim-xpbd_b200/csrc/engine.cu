@@ -266,7 +266,11 @@ public:
 	DBuf<float> ndist, nstiff, lam;
 	DBuf<unsigned int> ecode;        // neighbour and row (modulo 32) of each directed edge
 	DBuf<int> vol_off, vol_idx, rev_off, rev_idx, mat_type, vol_gs_order;
-	DBuf<int> vol_idx_s, rev_idx_s;  // the same lists, rows sorted along the curve
+	DBuf<int> rev_idx_s;             // the reverse lists, rows sorted along the curve
+	DBuf<int> vol_group, vol_pack;   // the member lists sorted so and packed for the solve (k_pack_members)
+	long long pack_groups = 0;       // groups of 16 in them
+	DBuf<int> vol_idx_s;             // unpacked again for the solve forms that set_volume_lanes asks for
+	int vol_idx_s_of = -1;           // generation it was unpacked from
 	DBuf<int> gather_order;          // gather group -> node: nodes of similar reverse-list length side by side
 	DBuf<float> det_rest, v_rest, rest_len, sigma_rest, lam_vol;
 	DBuf<float4> rec;
@@ -480,7 +484,7 @@ public:
 		obj_shift_valid = false;
 		pos_out3.release(); off.release(); nbr.release(); ndist.release(); nstiff.release(); lam.release(); ecode.release();
 		vol_off.release(); vol_idx.release(); rev_off.release(); rev_idx.release(); mat_type.release();
-		vol_idx_s.release(); rev_idx_s.release(); gather_order.release();
+		vol_idx_s.release(); rev_idx_s.release(); vol_group.release(); vol_pack.release(); vol_idx_s_of = -1; gather_order.release();
 		vol_gs_order.release(); det_rest.release(); v_rest.release(); rest_len.release(); sigma_rest.release();
 		lam_vol.release(); rec.release(); tiles.release(); gs_edge.release(); gs_rest.release(); gs_stiff.release(); gs_lam.release();
 		sc_keys.release(); sc_bucket.release(); sc_start.release(); sc_cursor.release(); sc_idx_sorted.release();
@@ -896,8 +900,20 @@ public:
 			build_mark(4);
 			const auto vs = sorted_rows(voff_i, vidx_i);
 			const auto rs = sorted_rows(roff_i, ridx_i);
-			CK(vol_idx_s.alloc(vs.size())); CK(rev_idx_s.alloc(rs.size()));
-			CK(cudaMemcpyAsync(vol_idx_s.p, vs.data(), sizeof(int) * vs.size(), cudaMemcpyHostToDevice, stream));
+			std::vector<int> group(n);
+			pack_groups = 0;
+			for (int r = 0; r < n; ++r) {
+				group[r] = (int)pack_groups;
+				pack_groups += (voff_i[r + 1] - voff_i[r] + 15) / 16;
+			}
+			DBuf<int> sorted;
+			CK(sorted.alloc(vs.size())); CK(rev_idx_s.alloc(rs.size()));
+			CK(vol_group.alloc(n)); CK(vol_pack.alloc(16 * (size_t)std::max<long long>(pack_groups, 1)));
+			CK(cudaMemcpyAsync(vol_group.p, group.data(), sizeof(int) * n, cudaMemcpyHostToDevice, stream));
+			CK(cudaMemcpyAsync(sorted.p, vs.data(), sizeof(int) * vs.size(), cudaMemcpyHostToDevice, stream));
+			dev::k_pack_members<<<blocks_for((long long)n * 32), kBlock, 0, stream>>>(n, vol_off.p, sorted.p, vol_group.p,
+				vol_pack.p, 1);
+			CK(cudaGetLastError());
 			CK(cudaMemcpyAsync(rev_idx_s.p, rs.data(), sizeof(int) * rs.size(), cudaMemcpyHostToDevice, stream));
 			{
 				std::vector<int> ord(n);
@@ -1451,6 +1467,33 @@ public:
 			(!S.use_volume || (vol_lanes() == 4 && S.lanes_a == 0 && gather_lanes() == 4)) && !S.use_angle && n > 0;
 	}
 
+	// the sorted lists unpacked, before a step that reads them
+	int ensure_sorted_members()
+	{
+		if (!S.use_volume || S.lanes_a == 0 || S.warp_mode != 0 || vol_idx_s_of == generation) return 0;
+		const size_t need = (size_t)std::max<long long>(arena ? m_cap : clusters.vol_off[n], 1);
+		if (vol_idx_s.n < need) CK(vol_idx_s.alloc(need));
+		dev::k_pack_members<<<blocks_for((long long)n * 32), kBlock, 0, stream>>>(n, vol_off.p, vol_idx_s.p, vol_group.p,
+			vol_pack.p, 0);
+		CK(cudaGetLastError());
+		vol_idx_s_of = generation;
+		return 0;
+	}
+
+	void enqueue_volume_solve(const float4* pin, int read_lam, int occ)
+	{
+		// two rounds of clusters per warp (its 3x3 work on 16 lanes) where that still leaves every
+		// SM its 40 resident warps: 148 us a launch at 1M against 164 with one round; with four
+		// rounds 147, but 49 against 43 at 200,000 (a last wave of few blocks)
+		const bool many = n >= 148 * 40 * 2 * dev::kSolveClusters;
+		const int rounds = many ? 2 : 1;
+		auto k = !many ? dev::k_volume_solve_warp<1, 5> : occ == 8 ? dev::k_volume_solve_warp<2, 8>
+			: occ == 6 ? dev::k_volume_solve_warp<2, 6> : dev::k_volume_solve_warp<2, 5>;
+		launch(ST_VOL_SOLVE, blocks_for(n, kBlock / 4 * rounds), dim3(kBlock), k, n, (const StepParams*)d_params, pin,
+			(const int*)vol_off.p, (const int*)vol_group.p, (const int4*)reinterpret_cast<const int4*>(vol_pack.p),
+			(const float*)det_rest.p, (const int*)mat_type.p, lam_vol.p, rec.p, recz(), read_lam);
+	}
+
 	void enqueue_tile_gather(const float4* pin, float4* pout)
 	{
 		if (tiles.count)
@@ -1486,7 +1529,7 @@ public:
 		A.pos_curr = pos_curr.p; A.pos_next = pos_next.p; A.pos_tmp = pos_tmp.p; A.vel = vel.p; A.lam_vol = lam_vol.p;
 		A.cshape = (cc || cg) ? c_shape.p : nullptr; A.crmax = cc ? c_rmax.p : nullptr; A.crg = cg ? c_rg.p : nullptr;
 		A.off = off.p; A.nbr = nbr.p; A.ndist = ndist.p; A.nstiff = nstiff.p; A.lam = lam.p;
-		A.vol_off = vol_off.p; A.vol_idx = vol_idx_s.p; A.mat_type = mat_type.p; A.rev_off = rev_off.p;
+		A.vol_off = vol_off.p; A.vol_group = vol_group.p; A.vol_pack = reinterpret_cast<const int4*>(vol_pack.p); A.mat_type = mat_type.p; A.rev_off = rev_off.p;
 		A.rev_idx = rev_idx_s.p; A.det_rest = det_rest.p; A.rest_len = rest_len.p; A.rec = rec.p; A.recz = recz();
 		A.tiles = tiles.tiles.p; A.tile_rows = tiles.rows.p; A.tile_words = tiles.words.p; A.tile_count = tiles.count;
 		A.list_rows = tiles.lists.p; A.list_count = tiles.list_count;
@@ -1586,11 +1629,7 @@ public:
 					const float4* cpin = pin;
 					if (la == 4 && S.lanes_a == 0)
 						// automatic: one pass over the members (any count), 4 lanes per cluster
-						launch(ST_VOL_SOLVE, blocks_for((long long)N * 4), B,
-							occ == 8 ? dev::k_volume_solve_occ<4, 8> : occ == 6 ? dev::k_volume_solve_occ<4, 6>
-							: dev::k_volume_solve_onepass<4>, N, dp, cpin,
-							(const int*)vol_off.p, (const int*)vol_idx_s.p, (const float*)det_rest.p,
-							(const int*)mat_type.p, lam_vol.p, rec.p, recz(), rl);
+						enqueue_volume_solve(cpin, rl, occ);
 					else if (la == 32)
 						launch(ST_VOL_SOLVE, blocks_for((long long)N * 32), B, dev::k_volume_solve_group<32, 8>, N, dp, cpin,
 							(const int*)vol_off.p, (const int*)vol_idx.p, (const float*)det_rest.p, (const int*)mat_type.p,
@@ -1689,7 +1728,7 @@ public:
 		}
 		if (S.use_distance && S.dist_gs && ensure_coloring()) return -1;
 		if (S.sc_enabled && ensure_selfcol()) return -1;
-		if (ensure_sc_object_buffers()) return -1;
+		if (ensure_sc_object_buffers() || ensure_sorted_members()) return -1;
 		const bool sc_limited_now = sc_limited();
 		if (upload_ext_colliders()) return -1;   // sets the object ranges fill_params reads
 		press_advance();
@@ -1853,7 +1892,7 @@ public:
 		int slot = -1, row0 = 0, rows = 0;
 		long long e0 = 0, ne = 0, m0 = 0, nm = 0, r0 = 0, nr = 0;
 		int t0 = 0, nt = 0, l0 = 0, nl = 0;      // tiles, rows in the list form, the tiles' words
-		long long w0 = 0, nw = 0;
+		long long w0 = 0, nw = 0, p0 = 0, np = 0;   // tile words, member groups
 		bool live = false;
 		std::vector<int> inv;   // session caller index -> row within the segment
 	};
@@ -1879,7 +1918,8 @@ public:
 		CK(mat_type.alloc(R)); CK(rec.alloc(3 * rec_rows())); CK(inv_mass_saved.alloc(R));
 		CK(off.alloc(R + 1)); CK(vol_off.alloc(R + 1)); CK(rev_off.alloc(R + 1));
 		CK(nbr.alloc((size_t)edges)); CK(ndist.alloc((size_t)edges)); CK(nstiff.alloc((size_t)edges));
-		CK(lam.alloc((size_t)edges)); CK(ecode.alloc((size_t)edges)); CK(vol_idx_s.alloc((size_t)members)); CK(rev_idx_s.alloc((size_t)rev));
+		CK(lam.alloc((size_t)edges)); CK(ecode.alloc((size_t)edges)); CK(rev_idx_s.alloc((size_t)rev));
+		CK(vol_group.alloc(R)); CK(vol_pack.alloc(16 * (((size_t)members + 15 * R) / 16 + 1)));   // padding: 15 a row at most
 		// a tile's words never outnumber its list entries (k_tile_build); at most a tile per 64 rows
 		CK(tiles.tiles.alloc(R / 64 + 1)); CK(tiles.rows.alloc(R)); CK(tiles.lists.alloc(R));
 		CK(tiles.words.alloc((size_t)std::min<long long>(rev, INT_MAX - 64)));
@@ -1965,6 +2005,7 @@ public:
 		g.slot = next_slot++;
 		g.row0 = rows_used; g.rows = rows;
 		g.e0 = e_used; g.ne = ne; g.m0 = m_used; g.nm = nm; g.r0 = r_used; g.nr = nr;
+		g.p0 = pack_groups; g.np = src.pack_groups;
 		g.live = true;
 		g.inv = src.inv;
 		const size_t r0 = (size_t)g.row0;
@@ -1978,7 +2019,8 @@ public:
 		if (copy_shift(src.d_perm.p, d_perm.p + r0, rows, g.row0) ||
 			copy_shift(src.off.p, off.p + r0, rows + 1, (int)g.e0) || copy_shift(src.nbr.p, nbr.p + g.e0, ne, g.row0) ||
 			copy_shift(src.vol_off.p, vol_off.p + r0, rows + 1, (int)g.m0) ||
-			copy_shift(src.vol_idx_s.p, vol_idx_s.p + g.m0, nm, g.row0) ||
+			copy_shift(src.vol_group.p, vol_group.p + r0, rows, (int)g.p0) ||
+			copy_shift(src.vol_pack.p, vol_pack.p + 16 * g.p0, 16 * g.np, g.row0) ||
 			copy_shift(src.rev_off.p, rev_off.p + r0, rows + 1, (int)g.r0) ||
 			copy_shift(src.rev_idx_s.p, rev_idx_s.p + g.r0, nr, g.row0))
 			return -1;
@@ -2009,6 +2051,7 @@ public:
 		}
 		rows_used += rows; e_used += ne; m_used += nm; r_used += nr;
 		tiles.count += g.nt; tiles.list_count += g.nl; tiles.words_used += g.nw;
+		pack_groups += g.np;
 		n = rows_used;
 		segs.push_back(std::move(g));
 		++generation;
@@ -2035,6 +2078,7 @@ public:
 			const ArenaSeg& b = segs.back();
 			rows_used = b.row0; e_used = b.e0; m_used = b.m0; r_used = b.r0;
 			tiles.count = b.t0; tiles.list_count = b.l0; tiles.words_used = b.w0;
+			pack_groups = b.p0;
 			segs.pop_back();
 		}
 		n = rows_used;
@@ -2051,7 +2095,7 @@ public:
 		for (const auto& g : segs)
 			if (g.live) {
 				stage_bytes = std::max(stage_bytes, std::max({ sizeof(float4) * (size_t)g.rows, sizeof(float) * 3 * (size_t)g.rows,
-					sizeof(int) * (size_t)(g.rows + 1), sizeof(int) * (size_t)g.ne, sizeof(int) * (size_t)g.nm,
+					sizeof(int) * (size_t)(g.rows + 1), sizeof(int) * (size_t)g.ne, sizeof(int) * 16 * (size_t)g.np,
 					sizeof(int) * (size_t)g.nr, sizeof(int) * (size_t)g.nw, sizeof(int) * (size_t)g.nl }));
 				stage_tiles = std::max<size_t>(stage_tiles, g.nt);
 			}
@@ -2073,7 +2117,7 @@ public:
 		};
 		std::vector<ArenaSeg> kept;
 		int rows = 0, nt = 0, nl = 0;
-		long long e = 0, m = 0, r = 0, words = 0;
+		long long e = 0, m = 0, r = 0, words = 0, groups = 0;
 		for (auto& g : segs) {
 			if (!g.live) continue;
 			const int dr = rows - g.row0;
@@ -2090,7 +2134,8 @@ public:
 					return -1;
 				if (move_shift(d_perm.p, a, b, k, dr) || move_shift(off.p, a, b, k + 1, (int)de) ||
 					move_shift(nbr.p, g.e0, e, g.ne, dr) || move_shift(vol_off.p, a, b, k + 1, (int)dm) ||
-					move_shift(vol_idx_s.p, g.m0, m, g.nm, dr) || move_shift(rev_off.p, a, b, k + 1, (int)drv) ||
+					move_shift(vol_group.p, a, b, k, (int)(groups - g.p0)) ||
+					move_shift(vol_pack.p, 16 * g.p0, 16 * groups, 16 * g.np, dr) || move_shift(rev_off.p, a, b, k + 1, (int)drv) ||
 					move_shift(rev_idx_s.p, g.r0, r, g.nr, dr))
 					return -1;
 				if (move_shift(tiles.rows.p, a, b, k, dr) || move_shift(tiles.lists.p, g.l0, nl, g.nl, dr)) return -1;
@@ -2106,16 +2151,17 @@ public:
 				dev::k_edge_codes<<<blocks_for(g.rows), kBlock, 0, stream>>>(g.rows, rows, off.p, nbr.p, ecode.p);
 				CK(cudaGetLastError());
 				g.l0 = nl;
-				g.t0 = nt; g.w0 = words;
+				g.t0 = nt; g.w0 = words; g.p0 = groups;
 				g.row0 = rows; g.e0 = e; g.m0 = m; g.r0 = r;
 			}
 			rows += g.rows; e += g.ne; m += g.nm; r += g.nr;
-			nt += g.nt; nl += g.nl; words += g.nw;
+			nt += g.nt; nl += g.nl; words += g.nw; groups += g.np;
 			kept.push_back(std::move(g));
 		}
 		segs.swap(kept);
 		rows_used = rows; e_used = e; m_used = m; r_used = r;
 		tiles.count = nt; tiles.list_count = nl; tiles.words_used = words;
+		pack_groups = groups;
 		n = rows_used;
 		++generation;
 		return sync();

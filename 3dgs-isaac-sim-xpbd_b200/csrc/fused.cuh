@@ -27,7 +27,8 @@ struct SubstepArgs {
 	const int *off, *nbr;
 	const float *ndist, *nstiff;
 	float* lam;
-	const int *vol_off, *vol_idx, *mat_type, *rev_off, *rev_idx;
+	const int *vol_off, *vol_group, *mat_type, *rev_off, *rev_idx;
+	const int4* vol_pack;
 	const VolTile* tiles;
 	const int* tile_rows;
 	const unsigned int* tile_words;
@@ -79,6 +80,7 @@ __global__ void __launch_bounds__(kBlock, 2) k_substep_fused(SubstepArgs A)
 {
 	extern __shared__ __align__(16) unsigned char slab[];   // kVtSmem
 	__shared__ unsigned int part[2][kVtThreads / 32];
+	__shared__ SolveSums sums[kBlock / 32];
 	DevCounters* ctr = A.ctr;
 	const long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
 	const long long nth = (long long)gridDim.x * blockDim.x;
@@ -101,9 +103,11 @@ __global__ void __launch_bounds__(kBlock, 2) k_substep_fused(SubstepArgs A)
 			float4* t = pin; pin = pout; pout = t;
 		}
 		if (A.use_volume) {
-			for (long long b = wbase; b < 4LL * n; b += nth)
-				solve_onepass_lane<4, false>(b + lane, n, P, pin, A.vol_off, A.vol_idx, A.det_rest, A.mat_type, A.lam_vol,
-					A.rec, A.recz, first ? 0 : 1);
+			for (long long b = wbase; b < n; b += nth) {
+				solve_warp<4, false>(sums[threadIdx.x >> 5], (int)b, n, P, pin, A.vol_off, A.vol_group, A.vol_pack, A.det_rest, A.mat_type,
+					A.lam_vol, A.rec, A.recz, first ? 0 : 1);
+				__syncwarp();
+			}
 			grid_barrier(ctr);
 			for (int t = blockIdx.x; t < A.tile_count; t += gridDim.x) {
 				tile_gather<false>(slab, part, n, P, pin, pout, A.tiles + t, A.tile_rows, A.tile_words, A.rev_off, A.rev_idx,

@@ -951,10 +951,15 @@ __global__ void __launch_bounds__(kSmemBlock) k_volume_solve_smem(int n, const S
 	store_record(rec, recz, idx, c, dl * gs, Sinv);
 }
 
-// Kernel A in one pass over the members (S lanes per cluster, members L, L+S, ... of
-// the curve-sorted list on lane L, two in flight per trip): each lane accumulates,
-// relative to the leader's position, the count, first and second moments of its
-// members and the same moments weighted by inverse mass.  The centred covariance
+// Kernel A in one pass over the members: a warp takes 8 R clusters, eight at a time on four
+// lanes each (members L, L + 4, ... of the curve-sorted list on lane L).  The lists are packed
+// in groups of sixteen, a lane's four members of a group side by side, so that it reads their
+// indices with one 128-bit load: eight clusters' lists lie in eight places, and a load of four
+// indices costs the same wavefronts as a load of one (two fifths of the kernel's, which it is
+// bound by).  The lanes sum, relative to the leader's position, the first and second moments of
+// the members; the sums wait in shared memory until a lane per cluster turns them into the
+// record, so that the 3x3 work, two fifths of the instructions when a lane in four did it,
+// runs on 8 R lanes at once.  The centred covariance
 //   Sigma = (1 / (m+1)) sum (q - c)(q - c)^T = sum d d^T / (m+1) - c' c'^T
 // (d = q - p_leader, c' = c - p_leader, the leader's d = 0) and the denominator
 //   sum w |g Sinv (q - c)|^2 = g^2 tr(Sinv^2 W),  W = sum w (d - c')(d - c')^T
@@ -963,150 +968,151 @@ __global__ void __launch_bounds__(kSmemBlock) k_volume_solve_smem(int n, const S
 // cancellation in the moment form small; the result equals the two-pass form
 // (forward.cu:8531-8664) to FP32 rounding.  The reference has the same leader-relative
 // moments in its optional one-pass warp kernel (forward.cu:8864-9033, warp mode 3).
-template <int S, bool NC>
-__device__ __forceinline__ void solve_onepass_lane(long long gtid, int n, const StepParams* __restrict__ P,
-	const float4* __restrict__ pin, const int* __restrict__ voff, const int* __restrict__ vidx,
+// The moments weighted by inverse mass are summed in a second pass over the members only when
+// their inverse masses differ (pinned members); otherwise they are w times the plain ones.
+// Measured (us per launch): 1,000,000 Gaussians 188 -> 148, 200,000 49 -> 43, 250,000 with
+// 128-member clusters 85 -> 67.  Five blocks per SM (48 registers): six spill, 169 us at 1M.
+constexpr int kSolveLanes = 4, kSolveClusters = 32 / kSolveLanes;   // at a time
+// per warp: d, d d^T (xx yy zz xy xz yz); w and whether it differs; the same sums weighted, w
+struct SolveSums { float plain[9][32], mass[32], mixed[32], weighted[10][32]; };
+template <int R, bool NC>
+__device__ __forceinline__ void solve_warp(SolveSums& S, int first, int n, const StepParams* __restrict__ P,
+	const float4* __restrict__ pin, const int* __restrict__ voff, const int* __restrict__ vgroup, const int4* __restrict__ vpack,
 	const float* __restrict__ det_rest, const int* __restrict__ mat_type, float* __restrict__ lam_vol,
 	float4* __restrict__ rec, float* __restrict__ recz, int read_lam)
 {
-	const int sl = (int)(gtid & (S - 1));
-	const int idx = (int)(gtid / S);
-	const bool in_range = idx < n;
-	bool valid = in_range && mat_type[idx] == 0;
-	int off = 0, cnt = 0;
-	float4 p4 = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-	if (valid) {
-		off = voff[idx];
-		cnt = voff[idx + 1] - off;
-		p4 = ldv<NC>(pin, idx);
-	}
-	const float3 pi = f3(p4);
+	const int lane = threadIdx.x & 31, sl = lane & (kSolveLanes - 1);
 	const float ims = P->inv_mass_scale;
-	// m[0..9]: count, d, d d^T (xx yy zz xy xz yz); m[10..19]: the same weighted by w.
-	// The weighted sums are formed in a second pass over the members only when their
-	// inverse masses differ; otherwise they are w times the plain ones
-	float m[20];
+#pragma unroll 1
+	for (int r = 0; r < R; ++r) {
+		const int slot = r * kSolveClusters + lane / kSolveLanes, idx = first + slot;
+		const int4* first_of = vpack;
+		int cnt = 0;
+		float3 pi = make_float3(0.0f, 0.0f, 0.0f);
+		if (idx < n && mat_type[idx] == 0) {
+			cnt = voff[idx + 1] - voff[idx];
+			first_of = vpack + 4 * (size_t)vgroup[idx] + sl;
+			pi = f3(ldv<NC>(pin, idx));
+		}
+		const int4* list = first_of;
+		float m[9] = { 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f };
+		float wmin = INFINITY, wmax = -INFINITY;
+		// f(offset from the leader, inverse mass) for this lane's members
+		auto members = [&](auto f) {
+			int4 next = cnt > 0 ? __ldg(list) : make_int4(0, 0, 0, 0);
+			for (int k = sl; k < cnt; k += 16) {   // members k, k + 4, k + 8, k + 12
+				const int j[4] = { next.x, next.y, next.z, next.w };
+				list += kSolveLanes;
+				if (k - sl + 16 < cnt) next = __ldg(list);
+				float4 q[4];
 #pragma unroll
-	for (int t = 0; t < 20; ++t) m[t] = 0.0f;
-	float wmin = INFINITY, wmax = -INFINITY;
-	auto add = [&](float4 q) {
-		const float dx = q.x - pi.x, dy = q.y - pi.y, dz = q.z - pi.z, w = q.w * ims;
-		m[0] += 1.0f; m[1] += dx; m[2] += dy; m[3] += dz;
-		m[4] += dx * dx; m[5] += dy * dy; m[6] += dz * dz; m[7] += dx * dy; m[8] += dx * dz; m[9] += dy * dz;
-		wmin = fminf(wmin, w); wmax = fmaxf(wmax, w);
-	};
-	auto add_w = [&](float4 q) {
-		const float dx = q.x - pi.x, dy = q.y - pi.y, dz = q.z - pi.z, w = q.w * ims;
-		m[10] += w; m[11] += w * dx; m[12] += w * dy; m[13] += w * dz;
-		m[14] += w * dx * dx; m[15] += w * dy * dy; m[16] += w * dz * dz;
-		m[17] += w * dx * dy; m[18] += w * dx * dz; m[19] += w * dy * dz;
-	};
-	int k = sl;
-	for (; k + S < cnt; k += 2 * S) {
-		const int j0 = __ldg(vidx + off + k), j1 = __ldg(vidx + off + k + S);
-		const bool ok0 = j0 >= 0 && j0 < n, ok1 = j1 >= 0 && j1 < n;
-		float4 q0 = make_float4(0.0f, 0.0f, 0.0f, 0.0f), q1 = q0;
-		if (ok0) q0 = ldv<NC>(pin, j0);
-		if (ok1) q1 = ldv<NC>(pin, j1);
-		if (ok0) add(q0);
-		if (ok1) add(q1);
-	}
-	if (k < cnt) {
-		const int j = __ldg(vidx + off + k);
-		if (j >= 0 && j < n) add(ldv<NC>(pin, j));
-	}
+				for (int t = 0; t < 4; ++t) q[t] = ldv<NC>(pin, j[t]);   // padding: the leader
 #pragma unroll
-	for (int t = 0; t < 10; ++t) m[t] = group_sum<S>(m[t]);
+				for (int t = 0; t < 4; ++t)
+					if (k + 4 * t < cnt) f(q[t].x - pi.x, q[t].y - pi.y, q[t].z - pi.z, q[t].w * ims);
+			}
+		};
+		members([&](float x, float y, float z, float w) {
+			m[0] += x; m[1] += y; m[2] += z;
+			m[3] += x * x; m[4] += y * y; m[5] += z * z; m[6] += x * y; m[7] += x * z; m[8] += y * z;
+			wmin = fminf(wmin, w); wmax = fmaxf(wmax, w);
+		});
 #pragma unroll
-	for (int o = 1; o < S; o <<= 1) {
-		wmin = fminf(wmin, __shfl_xor_sync(0xffffffffu, wmin, o, S));
-		wmax = fmaxf(wmax, __shfl_xor_sync(0xffffffffu, wmax, o, S));
-	}
-	const bool mixed = wmin < wmax;   // warp-uniform second pass (full-warp shuffles)
-	if (__any_sync(0xffffffffu, mixed)) {
-		if (mixed)
-			for (int k2 = sl; k2 < cnt; k2 += S) {
-				const int j = __ldg(vidx + off + k2);
-				if (j >= 0 && j < n) add_w(ldv<NC>(pin, j));
+		for (int q = 0; q < 9; ++q) m[q] = group_sum<kSolveLanes>(m[q]);
+#pragma unroll
+		for (int o = 1; o < kSolveLanes; o <<= 1) {
+			wmin = fminf(wmin, __shfl_xor_sync(0xffffffffu, wmin, o));
+			wmax = fmaxf(wmax, __shfl_xor_sync(0xffffffffu, wmax, o));
+		}
+		const bool mixed = wmin < wmax;
+		if (sl == 0) {
+#pragma unroll
+			for (int q = 0; q < 9; ++q) S.plain[q][slot] = m[q];
+			S.mass[slot] = wmin <= wmax ? wmin : 0.0f;   // 0: no member
+			S.mixed[slot] = mixed ? 1.0f : 0.0f;
+		}
+		if (__any_sync(0xffffffffu, mixed)) {
+			float v[10] = { 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f };   // w d, w d d^T, w
+			if (mixed) {
+				list = first_of;
+				members([&](float x, float y, float z, float w) {
+					v[0] += w * x; v[1] += w * y; v[2] += w * z;
+					v[3] += w * x * x; v[4] += w * y * y; v[5] += w * z * z;
+					v[6] += w * x * y; v[7] += w * x * z; v[8] += w * y * z;
+					v[9] += w;
+				});
 			}
 #pragma unroll
-		for (int t = 10; t < 20; ++t) m[t] = group_sum<S>(m[t]);
+			for (int q = 0; q < 10; ++q) {
+				v[q] = group_sum<kSolveLanes>(v[q]);
+				if (sl == 0) S.weighted[q][slot] = v[q];
+			}
+		}
 	}
-	if (!mixed) {   // one inverse mass over the members (or no member)
-		const float w0 = wmin <= wmax ? wmin : 0.0f;
+	__syncwarp();
+	// a lane per cluster
+	const int row = first + lane;
+	if (lane >= R * kSolveClusters || row >= n) return;
+	const int used = voff[row + 1] - voff[row];
+	const float4 p4 = ldv<NC>(pin, row);
+	float m[9];
 #pragma unroll
-		for (int t = 0; t < 10; ++t) m[10 + t] = w0 * m[t];
-	}
-	const int used = (int)(m[0] + 0.5f);
-	valid = valid && used >= 3;
+	for (int q = 0; q < 9; ++q) m[q] = S.plain[q][lane];
+	bool valid = mat_type[row] == 0 && used >= 3;
 	const float inv_n = 1.0f / (float)(used + 1);
-	const float cx = m[1] * inv_n, cy = m[2] * inv_n, cz = m[3] * inv_n;   // c - p_leader
-	const float3 c = make_float3(pi.x + cx, pi.y + cy, pi.z + cz);
-	M3 Sm;
-	Sm.m[0][0] = m[4] * inv_n - cx * cx;
-	Sm.m[1][1] = m[5] * inv_n - cy * cy;
-	Sm.m[2][2] = m[6] * inv_n - cz * cz;
-	Sm.m[0][1] = Sm.m[1][0] = m[7] * inv_n - cx * cy;
-	Sm.m[0][2] = Sm.m[2][0] = m[8] * inv_n - cx * cz;
-	Sm.m[1][2] = Sm.m[2][1] = m[9] * inv_n - cy * cz;
-	if (sl != 0 || !in_range) return;
+	const float cc[3] = { m[0] * inv_n, m[1] * inv_n, m[2] * inv_n };   // c - p_leader
 	float J = 1.0f, C = 0.0f;
 	M3 Sinv;
 	m3_zero(Sinv);
-	if (valid) valid = cluster_j_sinv(Sm, __ldg(det_rest + idx), J, C, Sinv);
-	if (!valid) { rec_invalidate(rec, idx); return; }
+	if (valid) {
+		M3 Sm;
+		Sm.m[0][0] = m[3] * inv_n - cc[0] * cc[0];
+		Sm.m[1][1] = m[4] * inv_n - cc[1] * cc[1];
+		Sm.m[2][2] = m[5] * inv_n - cc[2] * cc[2];
+		Sm.m[0][1] = Sm.m[1][0] = m[6] * inv_n - cc[0] * cc[1];
+		Sm.m[0][2] = Sm.m[2][0] = m[7] * inv_n - cc[0] * cc[2];
+		Sm.m[1][2] = Sm.m[2][1] = m[8] * inv_n - cc[1] * cc[2];
+		valid = cluster_j_sinv(Sm, __ldg(det_rest + row), J, C, Sinv);
+	}
+	if (!valid) { rec_invalidate(rec, row); return; }
 	const float gs = J * inv_n;
-	// W over members and leader (weight w_leader, d = 0)
-	const float wl = p4.w * ims;
-	const float ws = m[10] + wl;
-	float W[3][3];
-	const float wd[3] = { m[11], m[12], m[13] }, cc[3] = { cx, cy, cz };
-	const float wdd[3][3] = { { m[14], m[17], m[18] }, { m[17], m[15], m[19] }, { m[18], m[19], m[16] } };
-#pragma unroll
-	for (int a = 0; a < 3; ++a)
-#pragma unroll
-		for (int b = 0; b < 3; ++b) W[a][b] = wdd[a][b] - cc[a] * wd[b] - wd[a] * cc[b] + ws * cc[a] * cc[b];
+	const bool mixed = S.mixed[lane] != 0.0f;
+	const float w0 = S.mass[lane];
+	auto weighted = [&](int q) { return mixed ? S.weighted[q][lane] : w0 * (q < 9 ? m[q] : (float)used); };
+	const float wd[3] = { weighted(0), weighted(1), weighted(2) };
+	const float ws = weighted(9) + p4.w * ims;   // the leader: weight w, d = 0
 	// tr(Sinv^2 W) = sum_ab (Sinv^2)_ab W_ab
 	float dsum = 0.0f;
 #pragma unroll
-	for (int a = 0; a < 3; ++a)
-#pragma unroll
-		for (int b = 0; b < 3; ++b) {
-			const float s2 = Sinv.m[a][0] * Sinv.m[0][b] + Sinv.m[a][1] * Sinv.m[1][b] + Sinv.m[a][2] * Sinv.m[2][b];
-			dsum += s2 * W[a][b];
-		}
+	for (int q = 0; q < 6; ++q) {
+		const int a = q < 3 ? q : (q == 5 ? 1 : 0), b = q < 3 ? q : (q == 3 ? 1 : 2);
+		const float W = weighted(3 + q) - cc[a] * wd[b] - wd[a] * cc[b] + ws * cc[a] * cc[b];
+		const float s2 = Sinv.m[a][0] * Sinv.m[0][b] + Sinv.m[a][1] * Sinv.m[1][b] + Sinv.m[a][2] * Sinv.m[2][b];
+		dsum += (q < 3 ? 1.0f : 2.0f) * s2 * W;
+	}
 	const float denom = gs * gs * dsum;
 	const float dt = P->dt;
 	const float dt2 = fmaxf(dt * dt, 1e-8f);
 	const float alpha_t = P->vol_compliance / dt2;
 	const float den = denom + alpha_t;
-	if (!(den > 1e-12f)) { rec_invalidate(rec, idx); return; }
-	const float lam = read_lam ? lam_vol[idx] : 0.0f;
+	if (!(den > 1e-12f)) { rec_invalidate(rec, row); return; }
+	const float lam = read_lam ? lam_vol[row] : 0.0f;
 	const float dl = (-C - alpha_t * lam) / den;
-	if (!isfinite(dl)) { rec_invalidate(rec, idx); return; }
-	lam_vol[idx] = lam + dl;
-	store_record(rec, recz, idx, c, dl * gs, Sinv);
+	if (!isfinite(dl)) { rec_invalidate(rec, row); return; }
+	lam_vol[row] = lam + dl;
+	store_record(rec, recz, row, make_float3(p4.x + cc[0], p4.y + cc[1], p4.z + cc[2]), dl * gs, Sinv);
 }
-template <int S>
-__global__ void __launch_bounds__(kBlock) k_volume_solve_onepass(int n, const StepParams* __restrict__ P,
-	const float4* __restrict__ pin, const int* __restrict__ voff, const int* __restrict__ vidx,
+// compiled for MINB resident blocks per SM; the autotuner picks among the forms by timing
+template <int R, int MINB>
+__global__ void __launch_bounds__(kBlock, MINB) k_volume_solve_warp(int n, const StepParams* __restrict__ P,
+	const float4* __restrict__ pin, const int* __restrict__ voff, const int* __restrict__ vgroup, const int4* __restrict__ vpack,
 	const float* __restrict__ det_rest, const int* __restrict__ mat_type, float* __restrict__ lam_vol,
 	float4* __restrict__ rec, float* __restrict__ recz, int read_lam)
 {
-	solve_onepass_lane<S, true>((long long)blockIdx.x * blockDim.x + threadIdx.x, n, P, pin,
-		voff, vidx, det_rest, mat_type, lam_vol, rec, recz, read_lam);
-}
-// The volume solve compiled for MINB resident blocks per SM (fewer registers, more warps in
-// flight for its latency-bound gathers): the same per-item code, so the same results; the
-// autotuner picks among the forms by timing.
-template <int S, int MINB>
-__global__ void __launch_bounds__(kBlock, MINB) k_volume_solve_occ(int n, const StepParams* __restrict__ P,
-	const float4* __restrict__ pin, const int* __restrict__ voff, const int* __restrict__ vidx,
-	const float* __restrict__ det_rest, const int* __restrict__ mat_type, float* __restrict__ lam_vol,
-	float4* __restrict__ rec, float* __restrict__ recz, int read_lam)
-{
-	solve_onepass_lane<S, true>((long long)blockIdx.x * blockDim.x + threadIdx.x, n, P, pin,
-		voff, vidx, det_rest, mat_type, lam_vol, rec, recz, read_lam);
+	__shared__ SolveSums S[kBlock / 32];
+	const int warp = blockIdx.x * (kBlock / 32) + (threadIdx.x >> 5);
+	solve_warp<R, true>(S[threadIdx.x >> 5], warp * R * kSolveClusters, n, P, pin, voff, vgroup, vpack, det_rest, mat_type,
+		lam_vol, rec, recz, read_lam);
 }
 
 // Kernel A, one thread per cluster (forward.cu:8531-8664): sequential sums, leader first.
@@ -2909,6 +2915,23 @@ __global__ void k_edge_codes(int n, int row0, const int* __restrict__ off, const
 	if (i >= n) return;
 	const unsigned int r = (unsigned int)((row0 + i) & 31) << kCodeBits;
 	for (int e = off[row0 + i]; e < off[row0 + i + 1]; ++e) ecode[e] = r | (unsigned int)nbr[e];
+}
+
+// Member lists packed for the volume solve: row i's groups of sixteen start at group vgroup[i];
+// entry k of the list is word 4 (k & 3) + (k & 15) / 4 of group k / 16, padded with the row
+// itself.  pack: from the sorted lists; else back.  A warp per row.
+__global__ void __launch_bounds__(kBlock) k_pack_members(int n, const int* __restrict__ voff, int* __restrict__ sorted,
+	const int* __restrict__ vgroup, int* __restrict__ packed, int pack)
+{
+	const int row = (int)(((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
+	if (row >= n) return;
+	const int off = voff[row], cnt = voff[row + 1] - off;
+	int* p = packed + 16 * (size_t)vgroup[row];
+	for (int k = lane; k < ((cnt + 15) & ~15); k += 32) {
+		int* at = p + (k & ~15) + 4 * (k & 3) + ((k & 15) >> 2);
+		if (pack) *at = k < cnt ? sorted[off + k] : row;
+		else if (k < cnt) sorted[off + k] = *at;
+	}
 }
 
 // serving arena: copy of an index array with every non-negative entry shifted by delta
