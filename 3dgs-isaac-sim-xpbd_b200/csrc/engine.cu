@@ -1350,11 +1350,17 @@ public:
 	template <typename K, typename... A>
 	void launch(int stage, dim3 grid, dim3 block, K kernel, A... args)
 	{
-		launch_shared(stage, grid, block, 0, kernel, args...);
+		launch_as(stage, grid, block, 0, false, kernel, args...);
 	}
-	// the same with `shared` bytes of dynamic shared memory per block
+	// a kernel of the step's chain (chain_next / chain_wait in kernels.cuh), with `shared` bytes
+	// of dynamic shared memory per block
 	template <typename K, typename... A>
-	void launch_shared(int stage, dim3 grid, dim3 block, size_t shared, K kernel, A... args)
+	void launch_chain(int stage, dim3 grid, dim3 block, size_t shared, K kernel, A... args)
+	{
+		launch_as(stage, grid, block, shared, capturing && after_kernel, kernel, args...);
+	}
+	template <typename K, typename... A>
+	void launch_as(int stage, dim3 grid, dim3 block, size_t shared, bool chained, K kernel, A... args)
 	{
 		cudaEvent_t a = nullptr, b = nullptr;
 		if (profiling) {
@@ -1362,13 +1368,36 @@ public:
 			b = next_event();
 			cudaEventRecord(a, stream);
 		}
-		kernel<<<grid, block, shared, stream>>>(args...);
+		if (chained) {
+			cudaLaunchConfig_t cfg = {};
+			cfg.gridDim = grid;
+			cfg.blockDim = block;
+			cfg.dynamicSmemBytes = shared;
+			cfg.stream = stream;
+			cudaLaunchAttribute attr[1];
+			attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+			attr[0].val.programmaticStreamSerializationAllowed = 1;
+			cfg.attrs = attr;
+			cfg.numAttrs = 1;
+			cudaLaunchKernelEx(&cfg, kernel, args...);
+		}
+		else
+			kernel<<<grid, block, shared, stream>>>(args...);
+		after_kernel = true;
 		++launches;
 		if (profiling) {
 			cudaEventRecord(b, stream);
 			prof_records.push_back({ stage, a, b });
 		}
 	}
+	// a memset between the step's kernels; the next kernel is not chained to it
+	cudaError_t clear(void* p, size_t bytes)
+	{
+		after_kernel = false;
+		return cudaMemsetAsync(p, 0, bytes, stream);
+	}
+	bool capturing = false;          // the step is being captured
+	bool after_kernel = false;       // the last operation enqueued was a kernel
 	cudaEvent_t next_event()
 	{
 		if (event_next == event_pool.size()) {
@@ -1399,18 +1428,18 @@ public:
 		const unsigned mask = (unsigned)(sc_table - 1);
 		const bool near = sc_near_on();
 		// displacement max (and, for the near-pair grid, the box of the predicted positions)
-		launch(ST_SC_BUILD, dim3(std::min<unsigned>(G.x, 148u * 8u)), B, dev::k_sc_disp, N, (const float4*)pos_curr.p,
+		launch_chain(ST_SC_BUILD, dim3(std::min<unsigned>(G.x, 148u * 8u)), B, 0, dev::k_sc_disp, N, (const float4*)pos_curr.p,
 			(const float4*)pos_next.p, d_ctr, active, near ? 1 : 0);
-		launch(ST_SC_BUILD, dim3(1), dim3(1), dev::k_sc_setup, (const StepParams*)d_params, d_ctr);
+		launch_chain(ST_SC_BUILD, dim3(1), dim3(1), 0, dev::k_sc_setup, (const StepParams*)d_params, d_ctr);
 		if (!near || ref_structure) {
-			CK(cudaMemsetAsync(sc_bucket.p, 0, sc_bucket.bytes(), stream));
-			CK(cudaMemsetAsync(sc_cursor.p, 0, sc_cursor.bytes(), stream));
+			CK(clear(sc_bucket.p, sc_bucket.bytes()));
+			CK(clear(sc_cursor.p, sc_cursor.bytes()));
 			launch(ST_SC_BUILD, G, B, dev::k_sc_keys, N, (const float4*)pos_curr.p, (const DevCounters*)d_ctr, mask,
 				(unsigned)sc_table, sc_keys.p, sc_bucket.p, active);
-			launch(ST_SC_BUILD, dim3(nb), dim3(1024), dev::k_scan_blocks, (const int*)sc_bucket.p, sc_start.p, scan_n,
+			launch_chain(ST_SC_BUILD, dim3(nb), dim3(1024), 0, dev::k_scan_blocks, (const int*)sc_bucket.p, sc_start.p, scan_n,
 				sc_block_sums.p);
-			launch(ST_SC_BUILD, dim3(1), dim3(1024), dev::k_scan_sums, sc_block_sums.p, nb);
-			launch(ST_SC_BUILD, dim3(nb), dim3(1024), dev::k_scan_add, sc_start.p, scan_n, (const int*)sc_block_sums.p);
+			launch_chain(ST_SC_BUILD, dim3(1), dim3(1024), 0, dev::k_scan_sums, sc_block_sums.p, nb);
+			launch_chain(ST_SC_BUILD, dim3(nb), dim3(1024), 0, dev::k_scan_add, sc_start.p, scan_n, (const int*)sc_block_sums.p);
 			launch(ST_SC_BUILD, G, B, dev::k_sc_scatter, N, (const unsigned*)sc_keys.p, (const int*)sc_start.p,
 				sc_cursor.p, sc_idx_sorted.p);
 			launch(ST_SC_BUILD, blocks_for(buckets), B, dev::k_sc_order, buckets, (const int*)sc_start.p,
@@ -1419,17 +1448,17 @@ public:
 		if (near) {
 			// dense grid of the predicted positions: cell size, counts, starts, scatter
 			const int fscan = nf_cap + 1, fnb = (fscan + 1023) / 1024;
-			launch(ST_SC_BUILD, dim3(1), dim3(1), dev::k_sc_near_setup, (const StepParams*)d_params, d_ctr, nf_cap);
-			CK(cudaMemsetAsync(nf_bucket.p, 0, nf_bucket.bytes(), stream));
-			launch(ST_SC_BUILD, G, B, dev::k_sc_near_keys, N, (const float4*)pos_curr.p, (const float4*)pos_next.p,
+			launch_chain(ST_SC_BUILD, dim3(1), dim3(1), 0, dev::k_sc_near_setup, (const StepParams*)d_params, d_ctr, nf_cap);
+			CK(clear(nf_bucket.p, nf_bucket.bytes()));
+			launch_chain(ST_SC_BUILD, G, B, 0, dev::k_sc_near_keys, N, (const float4*)pos_curr.p, (const float4*)pos_next.p,
 				active, (const DevCounters*)d_ctr, nf_keys.p, nf_bucket.p);
-			launch(ST_SC_BUILD, dim3(fnb), dim3(1024), dev::k_scan_blocks, (const int*)nf_bucket.p, nf_start.p, fscan,
+			launch_chain(ST_SC_BUILD, dim3(fnb), dim3(1024), 0, dev::k_scan_blocks, (const int*)nf_bucket.p, nf_start.p, fscan,
 				sc_block_sums.p);
-			launch(ST_SC_BUILD, dim3(1), dim3(1024), dev::k_scan_sums, sc_block_sums.p, fnb);
-			launch(ST_SC_BUILD, dim3(fnb), dim3(1024), dev::k_scan_add, nf_start.p, fscan, (const int*)sc_block_sums.p);
-			launch(ST_SC_BUILD, G, B, dev::k_sc_near_scatter, N, (const unsigned*)nf_keys.p, (const int*)nf_start.p,
+			launch_chain(ST_SC_BUILD, dim3(1), dim3(1024), 0, dev::k_scan_sums, sc_block_sums.p, fnb);
+			launch_chain(ST_SC_BUILD, dim3(fnb), dim3(1024), 0, dev::k_scan_add, nf_start.p, fscan, (const int*)sc_block_sums.p);
+			launch_chain(ST_SC_BUILD, G, B, 0, dev::k_sc_near_scatter, N, (const unsigned*)nf_keys.p, (const int*)nf_start.p,
 				nf_bucket.p, (const float4*)pos_next.p, nf_p.p, sc_counts.p);
-			launch(ST_SC_BUILD, G, B, dev::k_sc_build_near, N, (const StepParams*)d_params, (const float4*)pos_curr.p,
+			launch_chain(ST_SC_BUILD, G, B, 0, dev::k_sc_build_near, N, (const StepParams*)d_params, (const float4*)pos_curr.p,
 				(const float4*)pos_next.p, (const float4*)pos_rest.p, active, (const int*)nf_start.p, mask,
 				(const float4*)nf_p.p, (const int*)d_perm.p, d_ctr, sc_contacts.p, sc_counts.p);
 			return 0;
@@ -1489,7 +1518,7 @@ public:
 		const int rounds = many ? 2 : 1;
 		auto k = !many ? dev::k_volume_solve_warp<1, 5> : occ == 8 ? dev::k_volume_solve_warp<2, 8>
 			: occ == 6 ? dev::k_volume_solve_warp<2, 6> : dev::k_volume_solve_warp<2, 5>;
-		launch(ST_VOL_SOLVE, blocks_for(n, kBlock / 4 * rounds), dim3(kBlock), k, n, (const StepParams*)d_params, pin,
+		launch_chain(ST_VOL_SOLVE, blocks_for(n, kBlock / 4 * rounds), dim3(kBlock), 0, k, n, (const StepParams*)d_params, pin,
 			(const int*)vol_off.p, (const int*)vol_group.p, (const int4*)reinterpret_cast<const int4*>(vol_pack.p),
 			(const float*)det_rest.p, (const int*)mat_type.p, lam_vol.p, rec.p, recz(), read_lam);
 	}
@@ -1497,12 +1526,12 @@ public:
 	void enqueue_tile_gather(const float4* pin, float4* pout)
 	{
 		if (tiles.count)
-			launch_shared(ST_VOL_GATHER, dim3(tiles.count), dim3(dev::kVtThreads), dev::kVtSmem, dev::k_tile_gather, n,
+			launch_chain(ST_VOL_GATHER, dim3(tiles.count), dim3(dev::kVtThreads), dev::kVtSmem, dev::k_tile_gather, n,
 				(const StepParams*)d_params, pin, pout, (const dev::VolTile*)tiles.tiles.p, (const int*)tiles.rows.p,
 				(const unsigned int*)tiles.words.p, (const int*)rev_off.p, (const int*)rev_idx_s.p, (const float4*)rec.p,
 				(const float*)recz(), (const float*)rest_len.p);
 		if (tiles.list_count)
-			launch(ST_VOL_GATHER, blocks_for((long long)tiles.list_count * 4), dim3(kBlock), dev::k_volume_gather_group<4>, n,
+			launch_chain(ST_VOL_GATHER, blocks_for((long long)tiles.list_count * 4), dim3(kBlock), 0, dev::k_volume_gather_group<4>, n,
 				(const StepParams*)d_params, pin, pout, (const int*)rev_off.p, (const int*)rev_idx_s.p, (const float4*)rec.p,
 				(const float*)recz(), (const float*)rest_len.p, (const int*)tiles.lists.p, tiles.list_count);
 	}
@@ -1536,7 +1565,7 @@ public:
 		A.pos_rest = pos_rest.p; A.shape_rest = shape_rest.p; A.shape_q = shape_q.p; A.ctr = d_ctr;
 		A.obj_id = d_obj_id.p; A.ext_kin = S.kin_ext.empty() ? nullptr : d_kin_ext.p; A.ext_range = d_kin_range.p;
 		A.pos_out3 = pos_out3.p; A.perm = d_perm.p;
-		CK(cudaMemsetAsync(d_ctr, 0, offsetof(DevCounters, jstats), stream));
+		CK(clear(d_ctr, offsetof(DevCounters, jstats)));
 		cudaLaunchConfig_t cfg = {};
 		cfg.gridDim = dim3(grid);
 		cfg.blockDim = dim3(kBlock);
@@ -1550,7 +1579,7 @@ public:
 		CK(cudaLaunchKernelEx(&cfg, dev::k_substep_fused, A));
 		++launches;
 		if (S.jstats) {
-			CK(cudaMemsetAsync(d_ctr->jstats, 0, sizeof(double) * 3, stream));
+			CK(clear(d_ctr->jstats, sizeof(double) * 3));
 			launch(ST_JSTATS, blocks_for(n), dim3(kBlock), dev::k_jstats, n, (const float4*)pos_curr.p,
 				(const int*)vol_off.p, (const int*)vol_idx.p, (const float*)det_rest.p, (const int*)mat_type.p,
 				(const float*)v_rest.p, d_ctr);
@@ -1567,12 +1596,12 @@ public:
 		const dim3 B(kBlock), G = blocks_for(N);
 		const dim3 GW = blocks_for((long long)N * 32);   // one warp per Gaussian / cluster
 		const bool sc = selfcol_on();
-		CK(cudaMemsetAsync(d_ctr, 0, offsetof(DevCounters, jstats), stream));
+		CK(clear(d_ctr, offsetof(DevCounters, jstats)));
 		const bool cc = contact_col(), cg = contact_ground();
 		const float4* cshape = (cc || cg) ? (const float4*)c_shape.p : (const float4*)nullptr;
 		const float* crmax = cc ? (const float*)c_rmax.p : (const float*)nullptr;
 		const float* crg = cg ? (const float*)c_rg.p : (const float*)nullptr;
-		launch(ST_PREDICT, G, B, dev::k_predict, N, (const StepParams*)d_params, (const float4*)pos_curr.p, pos_next.p,
+		launch_chain(ST_PREDICT, G, B, 0, dev::k_predict, N, (const StepParams*)d_params, (const float4*)pos_curr.p, pos_next.p,
 			vel.p, S.use_volume ? lam_vol.p : (float*)nullptr, cshape, cg ? c_rg.p : (float*)nullptr);
 		if (object_on()) enqueue_object_step(G, B);
 		const unsigned char* active = sc_limited() ? (const unsigned char*)sc_active.p : nullptr;
@@ -1582,7 +1611,7 @@ public:
 					(const float4*)pos_next.p, (const int*)d_obj_id.p, (const float*)obj_boxes.p,
 					(const float*)obj_disp.p, num_objects, sc_active.p, d_ctr);
 			if (enqueue_sc_build(active)) return -1;
-			if (obj_push()) CK(cudaMemsetAsync(sc_accum.p, 0, sc_accum.bytes(), stream));
+			if (obj_push()) CK(clear(sc_accum.p, sc_accum.bytes()));
 		}
 		float4* pin = pos_next.p;
 		float4* pout = pos_tmp.p;
@@ -1673,22 +1702,22 @@ public:
 			}
 			if (S.use_shape) {
 				if (S.shape_robust)
-					launch(ST_SHAPE, G, B, dev::k_shape_match<true>, N, (const StepParams*)d_params, (const float4*)pin,
+					launch_chain(ST_SHAPE, G, B, 0, dev::k_shape_match<true>, N, (const StepParams*)d_params, (const float4*)pin,
 						pout, (const float4*)pos_rest.p, (const int*)off.p, (const int*)nbr.p,
 						(const float4*)shape_rest.p, shape_q.p);
 				else
-					launch(ST_SHAPE, G, B, dev::k_shape_match<false>, N, (const StepParams*)d_params, (const float4*)pin,
+					launch_chain(ST_SHAPE, G, B, 0, dev::k_shape_match<false>, N, (const StepParams*)d_params, (const float4*)pin,
 						pout, (const float4*)pos_rest.p, (const int*)off.p, (const int*)nbr.p,
 						(const float4*)shape_rest.p, shape_q.p);
 				std::swap(pin, pout);
 			}
 			if (sc)
-				launch(ST_SC_SOLVE, G, B, dev::k_sc_solve, N, (const StepParams*)d_params, (const float4*)pin,
+				launch_chain(ST_SC_SOLVE, G, B, 0, dev::k_sc_solve, N, (const StepParams*)d_params, (const float4*)pin,
 					(const float4*)pos_curr.p, (const float4*)pos_rest.p, (const int*)sc_contacts.p,
 					(const int*)sc_counts.p, (const DevCounters*)d_ctr, sc_dp.p,
 					obj_push() ? sc_cross.p : (float4*)nullptr);
 			if (project)
-				launch(ST_PROJECT, G, B, dev::k_project, N, (const StepParams*)d_params, pin, (const float4*)pos_curr.p,
+				launch_chain(ST_PROJECT, G, B, 0, dev::k_project, N, (const StepParams*)d_params, pin, (const float4*)pos_curr.p,
 					sc ? (const int*)sc_counts.p : (const int*)nullptr, (const float4*)sc_dp.p, d_ctr, last ? 1 : 0,
 					(const int*)d_obj_id.p, S.kin_ext.empty() ? (const KinCollider*)nullptr : (const KinCollider*)d_kin_ext.p,
 					(const int2*)d_kin_range.p, (const float4*)sc_cross.p, obj_push() ? sc_accum.p : (float4*)nullptr,
@@ -1704,10 +1733,10 @@ public:
 			launch(ST_PROJECT, G, B, dev::k_obj_push_apply, N, (const StepParams*)d_params, (const int*)d_obj_id.p,
 				(const float4*)sc_accum.p, (const float*)push_T.p, (const DevCounters*)d_ctr, pin, crg);
 		}
-		launch(ST_VELOCITY, G, B, dev::k_velocity, N, (const StepParams*)d_params, pos_curr.p, (const float4*)pin,
+		launch_chain(ST_VELOCITY, G, B, 0, dev::k_velocity, N, (const StepParams*)d_params, pos_curr.p, (const float4*)pin,
 			vel.p, pos_out3.p, (const int*)d_perm.p, crg);
 		if (S.jstats) {
-			CK(cudaMemsetAsync(d_ctr->jstats, 0, sizeof(double) * 3, stream));
+			CK(clear(d_ctr->jstats, sizeof(double) * 3));
 			launch(ST_JSTATS, G, B, dev::k_jstats, N, (const float4*)pos_curr.p, (const int*)vol_off.p,
 				(const int*)vol_idx.p, (const float*)det_rest.p, (const int*)mat_type.p, (const float*)v_rest.p,
 				d_ctr);
@@ -1828,7 +1857,10 @@ public:
 		cudaGraph_t g = nullptr;
 		CK(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
 		const long long before = launches;
+		capturing = true;
+		after_kernel = false;
 		const int rc = form == 1 ? enqueue_step_fused() : enqueue_step(kFormOcc[form]);
+		capturing = false;
 		const cudaError_t ec = cudaStreamEndCapture(stream, &g);
 		if (rc) { if (g) cudaGraphDestroy(g); return -1; }
 		CK(ec);

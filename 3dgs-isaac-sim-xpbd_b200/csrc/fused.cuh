@@ -115,7 +115,7 @@ __global__ void __launch_bounds__(kBlock, 2) k_substep_fused(SubstepArgs A)
 				__syncthreads();
 			}
 			for (long long b = wbase; b < 4LL * A.list_count; b += nth)
-				gather_group_lane<4, false>((long long)ordered_node(A.list_rows, (int)(b + lane) / 4, A.list_count, n) * 4 +
+				gather_group_lane<4>((long long)ordered_node(A.list_rows, (int)(b + lane) / 4, A.list_count, n) * 4 +
 					(lane & 3), n, P, pin, pout, A.rev_off, A.rev_idx, A.rec, A.recz, A.rest_len);
 			grid_barrier(ctr);
 			float4* t = pin; pin = pout; pout = t;

@@ -17,6 +17,25 @@ namespace xpbd {
 namespace dev {
 
 // ---------------------------------------------------------------------------
+// The step's kernels are chained by programmatic dependent launch inside its CUDA graph: a
+// kernel lets the next one start (chain_next) and waits for the end of the one before, whose
+// writes are then visible (chain_wait), ahead of its first access to anything that a step's
+// kernel writes.  What only the upload wrote (topology, rest state, parameters) may be read
+// before the wait.  Every thread of a chained kernel that goes on waits, so the end of a
+// kernel implies the end of all before it.  Launched without the attribute both are no-ops.
+// A chained kernel runs beside the one whose results it reads, so those results never take
+// the read-only (non-coherent) path: ldv<false>, or pointers without __restrict__.
+// The long kernels call chain_next near their ends: the next kernel's blocks are placed where
+// there is room, and placed while an uneven kernel still fills half of the SMs they crowd the
+// other half (61,000 Gaussians, a frame: 2.80 ms unchained, 3.27 with chain_next first, 2.69
+// so).  Measured (ms per frame, unchained -> chained): 2,000 Gaussians 1.95 -> 1.86, 20,000
+// 2.26 -> 2.17, 200,000 with contact 6.15 -> 5.98, 1,000,000 23.3 -> 23.2.
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ void chain_next() { asm volatile("griddepcontrol.launch_dependents;"); }
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void chain() { chain_next(); chain_wait(); }
+
+// ---------------------------------------------------------------------------
 // small helpers (forward.cu:4949-4969; glm mat3 is column-major: m[col][row])
 // ---------------------------------------------------------------------------
 struct M3 { float m[3][3]; };
@@ -258,7 +277,7 @@ __global__ void __launch_bounds__(kBlock) k_contact_pack(int n, const float* __r
 // written per Gaussian (+32 B read, 4 B written with ground contact shapes).
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ void predict_row(int i, int n, const StepParams* __restrict__ P,
-	const float4* __restrict__ pos_curr, float4* __restrict__ pos_next, float4* __restrict__ vel,
+	const float4* pos_curr, float4* __restrict__ pos_next, float4* __restrict__ vel,
 	float* __restrict__ lam_vol, const float4* __restrict__ cshape, float* __restrict__ crg)
 {
 	if (i >= n) return;
@@ -280,9 +299,10 @@ __device__ __forceinline__ void predict_row(int i, int n, const StepParams* __re
 	}
 }
 __global__ void __launch_bounds__(kBlock) k_predict(int n, const StepParams* __restrict__ P,
-	const float4* __restrict__ pos_curr, float4* __restrict__ pos_next, float4* __restrict__ vel,
+	const float4* pos_curr, float4* __restrict__ pos_next, float4* __restrict__ vel,
 	float* __restrict__ lam_vol, const float4* __restrict__ cshape, float* __restrict__ crg)
 {
+	chain();
 	predict_row(blockIdx.x * blockDim.x + threadIdx.x, n, P, pos_curr, pos_next, vel, lam_vol, cshape, crg);
 }
 
@@ -415,10 +435,11 @@ __global__ void __launch_bounds__(kDistWarps * 32) k_distance_jacobi(int n, cons
 	if (row0 >= n) return;
 	const int row = row0 + lane;
 	const int e0 = off[min(row, n)], e1 = off[min(row + 1, n)];
-	float4 p4 = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-	if (row < n) p4 = ld4(pin, row);
-	s_row[w][lane] = p4;
 	const int begin = __shfl_sync(0xffffffffu, e0, 0), end = __shfl_sync(0xffffffffu, e1, 31);
+	chain_wait();
+	float4 p4 = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+	if (row < n) p4 = ldv<false>(pin, row);
+	s_row[w][lane] = p4;
 	__syncwarp();
 	const float ims = P->inv_mass_scale;
 	EdgeCompliance alpha(P);
@@ -441,7 +462,7 @@ __global__ void __launch_bounds__(kDistWarps * 32) k_distance_jacobi(int n, cons
 				}
 #pragma unroll
 			for (int t = 0; t < kDistTrips; ++t)
-				if (at + 32 * t < w1) q[t] = ld4(pin, (int)(code[t] & ((1u << kCodeBits) - 1u)));
+				if (at + 32 * t < w1) q[t] = ldv<false>(pin, (int)(code[t] & ((1u << kCodeBits) - 1u)));
 #pragma unroll
 			for (int t = 0; t < kDistTrips; ++t)
 				if (at + 32 * t < w1) {
@@ -461,6 +482,7 @@ __global__ void __launch_bounds__(kDistWarps * 32) k_distance_jacobi(int n, cons
 		for (int e = max(e0, w0); e < min(e1, w1); ++e) sum = add4(sum, s_corr[w][e - w0]);
 		__syncwarp();
 	}
+	chain_next();
 	if (row >= n) return;
 	const float3 out = sum.w > 0.0f ? distance_move(f3(p4), sum, P->under_relax) : f3(p4);
 	pout[row] = make_float4(out.x, out.y, out.z, p4.w);
@@ -975,7 +997,7 @@ __global__ void __launch_bounds__(kSmemBlock) k_volume_solve_smem(int n, const S
 constexpr int kSolveLanes = 4, kSolveClusters = 32 / kSolveLanes;   // at a time
 // per warp: d, d d^T (xx yy zz xy xz yz); w and whether it differs; the same sums weighted, w
 struct SolveSums { float plain[9][32], mass[32], mixed[32], weighted[10][32]; };
-template <int R, bool NC>
+template <int R, bool CHAIN>
 __device__ __forceinline__ void solve_warp(SolveSums& S, int first, int n, const StepParams* __restrict__ P,
 	const float4* __restrict__ pin, const int* __restrict__ voff, const int* __restrict__ vgroup, const int4* __restrict__ vpack,
 	const float* __restrict__ det_rest, const int* __restrict__ mat_type, float* __restrict__ lam_vol,
@@ -992,21 +1014,22 @@ __device__ __forceinline__ void solve_warp(SolveSums& S, int first, int n, const
 		if (idx < n && mat_type[idx] == 0) {
 			cnt = voff[idx + 1] - voff[idx];
 			first_of = vpack + 4 * (size_t)vgroup[idx] + sl;
-			pi = f3(ldv<NC>(pin, idx));
 		}
 		const int4* list = first_of;
+		int4 next = cnt > 0 ? __ldg(list) : make_int4(0, 0, 0, 0);
+		if (CHAIN && r == 0) chain_wait();
+		if (cnt > 0) pi = f3(ldv<false>(pin, idx));
 		float m[9] = { 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f };
 		float wmin = INFINITY, wmax = -INFINITY;
 		// f(offset from the leader, inverse mass) for this lane's members
 		auto members = [&](auto f) {
-			int4 next = cnt > 0 ? __ldg(list) : make_int4(0, 0, 0, 0);
 			for (int k = sl; k < cnt; k += 16) {   // members k, k + 4, k + 8, k + 12
 				const int j[4] = { next.x, next.y, next.z, next.w };
 				list += kSolveLanes;
 				if (k - sl + 16 < cnt) next = __ldg(list);
 				float4 q[4];
 #pragma unroll
-				for (int t = 0; t < 4; ++t) q[t] = ldv<NC>(pin, j[t]);   // padding: the leader
+				for (int t = 0; t < 4; ++t) q[t] = ldv<false>(pin, j[t]);   // padding: the leader
 #pragma unroll
 				for (int t = 0; t < 4; ++t)
 					if (k + 4 * t < cnt) f(q[t].x - pi.x, q[t].y - pi.y, q[t].z - pi.z, q[t].w * ims);
@@ -1035,6 +1058,7 @@ __device__ __forceinline__ void solve_warp(SolveSums& S, int first, int n, const
 			float v[10] = { 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f };   // w d, w d d^T, w
 			if (mixed) {
 				list = first_of;
+				next = __ldg(list);
 				members([&](float x, float y, float z, float w) {
 					v[0] += w * x; v[1] += w * y; v[2] += w * z;
 					v[3] += w * x * x; v[4] += w * y * y; v[5] += w * z * z;
@@ -1052,9 +1076,10 @@ __device__ __forceinline__ void solve_warp(SolveSums& S, int first, int n, const
 	__syncwarp();
 	// a lane per cluster
 	const int row = first + lane;
+	if (CHAIN) chain_next();
 	if (lane >= R * kSolveClusters || row >= n) return;
 	const int used = voff[row + 1] - voff[row];
-	const float4 p4 = ldv<NC>(pin, row);
+	const float4 p4 = ldv<false>(pin, row);
 	float m[9];
 #pragma unroll
 	for (int q = 0; q < 9; ++q) m[q] = S.plain[q][lane];
@@ -1219,7 +1244,7 @@ __device__ __forceinline__ float3 gather_finish(float3 pi, float3 avg, float rl,
 // Kernel B on groups of S lanes per node (forward.cu:9262-9323 with S = 32): mean over
 // the clusters that contain the node, step clamp 0.25 restLen, under-relaxation.  Reads
 // per node: h reverse indices + h gathered 36-byte records (L2-resident).
-template <int S, bool NC>
+template <int S>
 __device__ __forceinline__ void gather_group_lane(long long gtid, int n, const StepParams* __restrict__ P,
 	const float4* __restrict__ pin, float4* __restrict__ pout, const int* __restrict__ roff,
 	const int* __restrict__ ridx, const float4* __restrict__ rec, const float* __restrict__ recz,
@@ -1232,7 +1257,7 @@ __device__ __forceinline__ void gather_group_lane(long long gtid, int n, const S
 	int off = 0, cnt = 0;
 	float wi = 0.0f;
 	if (in_range) {
-		p4 = ldv<NC>(pin, idx);
+		p4 = ldv<false>(pin, idx);
 		wi = p4.w * P->inv_mass_scale;
 		if (wi > 0.0f) {
 			off = roff[idx];
@@ -1252,8 +1277,8 @@ __device__ __forceinline__ void gather_group_lane(long long gtid, int n, const S
 		float4 a0 = make_float4(0.0f, 0.0f, 0.0f, 0.0f), b0 = a0, a1 = a0, b1 = a0;
 		float z0 = 0.0f, z1 = 0.0f;
 		const float* cz = recz;
-		if (ok0) { ld_rec<NC>(rec, i0, a0, b0); z0 = ldv<NC>(cz, i0); }
-		if (ok1) { ld_rec<NC>(rec, i1, a1, b1); z1 = ldv<NC>(cz, i1); }
+		if (ok0) { ld_rec<false>(rec, i0, a0, b0); z0 = ldv<false>(cz, i0); }
+		if (ok1) { ld_rec<false>(rec, i1, a1, b1); z1 = ldv<false>(cz, i1); }
 		float3 dp;
 		if (ok0 && gather_rec(a0, b0, z0, pi, wi, dp)) { sum = add3(sum, dp); ++received; }
 		if (ok1 && gather_rec(a1, b1, z1, pi, wi, dp)) { sum = add3(sum, dp); ++received; }
@@ -1262,8 +1287,8 @@ __device__ __forceinline__ void gather_group_lane(long long gtid, int n, const S
 		const int i = __ldg(ridx + off + k);
 		float3 dp;
 		float4 a = make_float4(0.0f, 0.0f, 0.0f, 0.0f), b = a;
-		if (i >= 0 && i < n) ld_rec<NC>(rec, i, a, b);
-		if (i >= 0 && i < n && gather_rec(a, b, ldv<NC>(recz, i), pi, wi, dp)) {
+		if (i >= 0 && i < n) ld_rec<false>(rec, i, a, b);
+		if (i >= 0 && i < n && gather_rec(a, b, ldv<false>(recz, i), pi, wi, dp)) {
 			sum = add3(sum, dp);
 			++received;
 		}
@@ -1292,8 +1317,9 @@ __global__ void __launch_bounds__(kBlock, S == 4 ? 6 : 1) k_volume_gather_group(
 	const int* __restrict__ ridx, const float4* __restrict__ rec, const float* __restrict__ recz,
 	const float* __restrict__ rest_len, const int* __restrict__ order, int count)
 {
+	chain();
 	const long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-	gather_group_lane<S, true>((long long)ordered_node(order, (int)(g / S), count, n) * S + (g & (S - 1)), n, P, pin,
+	gather_group_lane<S>((long long)ordered_node(order, (int)(g / S), count, n) * S + (g & (S - 1)), n, P, pin,
 		pout, roff, ridx, rec, recz, rest_len);
 }
 
@@ -1809,14 +1835,14 @@ __global__ void __launch_bounds__(kBlock) k_shape_rest(int n, const float4* __re
 // {i} + 1-ring, normalised, rotation by polar decomposition (to FP64 rounding when ROBUST,
 // else float), goal projection.  The rest-only terms come from k_shape_rest.  at(e): the
 // neighbour of edge e.
-template <bool ROBUST, bool NC, class Neighbour>
+template <bool ROBUST, bool CHAIN, class Neighbour>
 __device__ __forceinline__ void shape_row(int idx, int n, const StepParams* __restrict__ P,
 	const float4* __restrict__ pin, float4* __restrict__ pout, const float4* __restrict__ rest,
 	const int* __restrict__ off, const Neighbour& at, const float4* __restrict__ shape_rest,
 	float4* __restrict__ shape_q)
 {
 	if (idx >= n) return;
-	const float4 p4 = ldv<NC>(pin, idx);
+	const float4 p4 = ldv<false>(pin, idx);
 	const float3 pi = f3(p4);
 	const float wi = p4.w * P->inv_mass_scale;
 	if (wi <= 0.0f) { pout[idx] = p4; return; }
@@ -1851,14 +1877,14 @@ __device__ __forceinline__ void shape_row(int idx, int n, const StepParams* __re
 		const int j0 = at(e), j1 = at(e + 1);
 		const bool ok0 = j0 >= 0 && j0 < n, ok1 = j1 >= 0 && j1 < n;
 		float4 q0 = make_float4(0.0f, 0.0f, 0.0f, 0.0f), q1 = q0, r0 = q0, r1 = q0;
-		if (ok0) { q0 = ldv<NC>(pin, j0); r0 = ld4(rest, j0); }
-		if (ok1) { q1 = ldv<NC>(pin, j1); r1 = ld4(rest, j1); }
+		if (ok0) { q0 = ldv<false>(pin, j0); r0 = ld4(rest, j0); }
+		if (ok1) { q1 = ldv<false>(pin, j1); r1 = ld4(rest, j1); }
 		if (ok0) add(q0, r0);
 		if (ok1) add(q1, r1);
 	}
 	if (e < e1) {
 		const int j = at(e);
-		if (j >= 0 && j < n) add(ldv<NC>(pin, j), ld4(rest, j));
+		if (j >= 0 && j < n) add(ldv<false>(pin, j), ld4(rest, j));
 	}
 	const float3 com_curr = mul3(sq, sr.w);
 	const float3 cq = sub3(com_curr, pi), cr = sub3(com_rest, ri);
@@ -1872,6 +1898,7 @@ __device__ __forceinline__ void shape_row(int idx, int n, const StepParams* __re
 		for (int r = 0; r < 3; ++r) a_norm_sq += A.m[c][r] * A.m[c][r];
 	const float a_norm = sqrtf(a_norm_sq);
 	if (!isfinite(a_norm) || a_norm < 1e-8f) { pout[idx] = p4; return; }
+	if (CHAIN) chain_next();
 	const float a_inv = 1.0f / a_norm;
 #pragma unroll
 	for (int c = 0; c < 3; ++c)
@@ -1924,6 +1951,7 @@ __global__ void __launch_bounds__(kBlock, 3) k_shape_match(int n, const StepPara
 	if (held)
 		for (int e = begin + lane; e < end; e += 32) window[e - begin] = __ldg(nbr + e);
 	__syncwarp();
+	chain_wait();
 	auto at = [&](int e) { return held ? window[e - begin] : __ldg(nbr + e); };
 	shape_row<ROBUST, true>(row0 + lane, n, P, pin, pout, rest, off, at, shape_rest, shape_q);
 }
@@ -1937,11 +1965,11 @@ __global__ void __launch_bounds__(kBlock, 3) k_shape_match(int n, const StepPara
 // ground contact shapes (crg non-null) the plane is offset by the support radius.
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ void project_row(int idx, int n, const StepParams* __restrict__ P, float4* __restrict__ pos,
-	const float4* __restrict__ pos_start, const int* __restrict__ sc_count, const float4* __restrict__ sc_dp,
+	const float4* pos_start, const int* sc_count, const float4* sc_dp,
 	DevCounters* __restrict__ ctr, int count_hits, const int* __restrict__ obj_id,
-	const KinCollider* __restrict__ ext_kin, const int2* __restrict__ ext_range, const float4* __restrict__ sc_dp_cross,
+	const KinCollider* __restrict__ ext_kin, const int2* __restrict__ ext_range, const float4* sc_dp_cross,
 	float4* __restrict__ sc_accum, const float4* __restrict__ cshape, const float* __restrict__ crmax,
-	const float* __restrict__ crg)
+	const float* crg)
 {
 	if (idx >= n) return;
 	float4 p4 = pos[idx];
@@ -2078,12 +2106,13 @@ __device__ __forceinline__ void project_row(int idx, int n, const StepParams* __
 	if (moved) pos[idx] = p4;
 }
 __global__ void __launch_bounds__(kBlock) k_project(int n, const StepParams* __restrict__ P, float4* __restrict__ pos,
-	const float4* __restrict__ pos_start, const int* __restrict__ sc_count, const float4* __restrict__ sc_dp,
+	const float4* pos_start, const int* sc_count, const float4* sc_dp,
 	DevCounters* __restrict__ ctr, int count_hits, const int* __restrict__ obj_id,
-	const KinCollider* __restrict__ ext_kin, const int2* __restrict__ ext_range, const float4* __restrict__ sc_dp_cross,
+	const KinCollider* __restrict__ ext_kin, const int2* __restrict__ ext_range, const float4* sc_dp_cross,
 	float4* __restrict__ sc_accum, const float4* __restrict__ cshape, const float* __restrict__ crmax,
-	const float* __restrict__ crg)
+	const float* crg)
 {
+	chain();
 	project_row(blockIdx.x * blockDim.x + threadIdx.x, n, P, pos, pos_start, sc_count, sc_dp, ctr, count_hits, obj_id,
 		ext_kin, ext_range, sc_dp_cross, sc_accum, cshape, crmax, crg);
 }
@@ -2093,8 +2122,8 @@ __global__ void __launch_bounds__(kBlock) k_project(int n, const StepParams* __r
 // also refreshes the caller-layout float3 position mirror.
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ void velocity_row(int idx, int n, const StepParams* __restrict__ P,
-	float4* __restrict__ pos_curr, const float4* __restrict__ pfinal, float4* __restrict__ vel,
-	float* __restrict__ pos_out3, const int* __restrict__ perm, const float* __restrict__ crg)
+	float4* __restrict__ pos_curr, const float4* pfinal, float4* __restrict__ vel,
+	float* __restrict__ pos_out3, const int* __restrict__ perm, const float* crg)
 {
 	if (idx >= n) return;
 	const float4 x4 = pos_curr[idx];
@@ -2154,9 +2183,10 @@ __device__ __forceinline__ void velocity_row(int idx, int n, const StepParams* _
 	}
 }
 __global__ void __launch_bounds__(kBlock) k_velocity(int n, const StepParams* __restrict__ P,
-	float4* __restrict__ pos_curr, const float4* __restrict__ pfinal, float4* __restrict__ vel,
-	float* __restrict__ pos_out3, const int* __restrict__ perm, const float* __restrict__ crg)
+	float4* __restrict__ pos_curr, const float4* pfinal, float4* __restrict__ vel,
+	float* __restrict__ pos_out3, const int* __restrict__ perm, const float* crg)
 {
+	chain();
 	velocity_row(blockIdx.x * blockDim.x + threadIdx.x, n, P, pos_curr, pfinal, vel, pos_out3, perm, crg);
 }
 
@@ -2233,9 +2263,10 @@ __device__ __forceinline__ float f_unorder(unsigned int u)
 // and predicted position finite) for the near-pair grid: order-preserving images, the
 // minimum complemented, so that both ends are atomicMax on zero-initialised counters.
 // Grid-stride over the particles, one set of atomics per block.
-__global__ void __launch_bounds__(kBlock) k_sc_disp(int n, const float4* __restrict__ x, const float4* __restrict__ p,
-	DevCounters* __restrict__ ctr, const unsigned char* __restrict__ active, int bounds)
+__global__ void __launch_bounds__(kBlock) k_sc_disp(int n, const float4* x, const float4* p,
+	DevCounters* __restrict__ ctr, const unsigned char* active, int bounds)
 {
+	chain();
 	unsigned int m[7] = { 0u, 0u, 0u, 0u, 0u, 0u, 0u };   // disp^2 bits, lo x y z, hi x y z
 	for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
 		if (active && !active[i]) continue;
@@ -2273,6 +2304,7 @@ __global__ void __launch_bounds__(kBlock) k_sc_disp(int n, const float4* __restr
 // cell size = search + 2 max|p - x|, capped (forward.cu:11818-11831)
 __global__ void k_sc_setup(const StepParams* __restrict__ P, DevCounters* __restrict__ ctr)
 {
+	chain();
 	const float md2 = __uint_as_float(ctr->sc_max_disp2_bits);
 	const float md = (isfinite(md2) && md2 > 0.0f) ? sqrtf(md2) : 0.0f;
 	float reach = P->sc_search + 2.0f * md;
@@ -2299,9 +2331,10 @@ __global__ void __launch_bounds__(kBlock) k_sc_keys(int n, const float4* __restr
 }
 
 // exclusive scan of bucket counts, three phases (block sums, scan of sums, apply)
-__global__ void __launch_bounds__(1024) k_scan_blocks(const int* __restrict__ in, int* __restrict__ out, int n,
+__global__ void __launch_bounds__(1024) k_scan_blocks(const int* in, int* __restrict__ out, int n,
 	int* __restrict__ block_sums)
 {
+	chain();
 	__shared__ int s[1024];
 	const int i = blockIdx.x * 1024 + threadIdx.x;
 	const int v = (i < n) ? in[i] : 0;
@@ -2318,6 +2351,7 @@ __global__ void __launch_bounds__(1024) k_scan_blocks(const int* __restrict__ in
 }
 __global__ void __launch_bounds__(1024) k_scan_sums(int* __restrict__ sums, int nb)
 {
+	chain();
 	// single block, sequential chunks of 1024
 	__shared__ int s[1024];
 	__shared__ int carry;
@@ -2340,8 +2374,9 @@ __global__ void __launch_bounds__(1024) k_scan_sums(int* __restrict__ sums, int 
 		__syncthreads();
 	}
 }
-__global__ void __launch_bounds__(1024) k_scan_add(int* __restrict__ out, int n, const int* __restrict__ sums)
+__global__ void __launch_bounds__(1024) k_scan_add(int* __restrict__ out, int n, const int* sums)
 {
+	chain();
 	const int i = blockIdx.x * 1024 + threadIdx.x;
 	if (i < n) out[i] += sums[blockIdx.x];
 }
@@ -2572,6 +2607,7 @@ __device__ __forceinline__ bool sc_near_member(const float4& x, const float4& p,
 // and cells per axis
 __global__ void k_sc_near_setup(const StepParams* __restrict__ P, DevCounters* __restrict__ ctr, int cap)
 {
+	chain();
 	float cell = P->sc_search * kNearCellScale;
 	float lo[3] = { 0.0f, 0.0f, 0.0f }, ext[3] = { 0.0f, 0.0f, 0.0f };
 	if (ctr->nb_hi[0] | ctr->nb_hi[1] | ctr->nb_hi[2]) {
@@ -2606,10 +2642,11 @@ __device__ __forceinline__ int sc_near_axis(float v, float o, float inv, int dim
 // dense-grid keys (cell index, x fastest) of the grid's particles and cell counts;
 // particles outside the reference's grid (inactive, or a start / predicted position not
 // finite) are left out
-__global__ void __launch_bounds__(kBlock) k_sc_near_keys(int n, const float4* __restrict__ X,
-	const float4* __restrict__ Pp, const unsigned char* __restrict__ active, const DevCounters* __restrict__ ctr,
+__global__ void __launch_bounds__(kBlock) k_sc_near_keys(int n, const float4* X,
+	const float4* Pp, const unsigned char* active, const DevCounters* ctr,
 	unsigned int* __restrict__ keys, int* __restrict__ bucket)
 {
+	chain();
 	const int i = blockIdx.x * blockDim.x + threadIdx.x;
 	if (i >= n) return;
 	const float4 x = X[i], p = Pp[i];
@@ -2629,10 +2666,11 @@ __global__ void __launch_bounds__(kBlock) k_sc_near_keys(int n, const float4* __
 // scatter predicted position + index into the cells (order within a cell is free: the
 // lists are ordered by key afterwards); leaves the cell counts at zero; a particle outside
 // the grid gets its empty candidate list here
-__global__ void __launch_bounds__(kBlock) k_sc_near_scatter(int n, const unsigned int* __restrict__ keys,
-	const int* __restrict__ start, int* __restrict__ bucket, const float4* __restrict__ Pp, float4* __restrict__ fp,
+__global__ void __launch_bounds__(kBlock) k_sc_near_scatter(int n, const unsigned int* keys,
+	const int* start, int* __restrict__ bucket, const float4* Pp, float4* __restrict__ fp,
 	int* __restrict__ counts)
 {
+	chain();
 	const int i = blockIdx.x * blockDim.x + threadIdx.x;
 	if (i >= n) return;
 	const unsigned int k = keys[i];
@@ -2661,11 +2699,12 @@ __device__ __forceinline__ unsigned long long sc_near_key(const Hash27& Href, fl
 // six resident blocks per SM: the row scans are latency bound; the spills fall in the
 // rarely used key batches
 __global__ void __launch_bounds__(kBlock, 6) k_sc_build_near(int n, const StepParams* __restrict__ P,
-	const float4* __restrict__ X, const float4* __restrict__ Pp, const float4* __restrict__ rest,
-	const unsigned char* __restrict__ active, const int* __restrict__ start_f, unsigned int mask,
-	const float4* __restrict__ fp, const int* __restrict__ perm, DevCounters* __restrict__ ctr,
+	const float4* X, const float4* Pp, const float4* __restrict__ rest,
+	const unsigned char* active, const int* start_f, unsigned int mask,
+	const float4* fp, const int* __restrict__ perm, DevCounters* __restrict__ ctr,
 	int* __restrict__ contacts, int* __restrict__ counts)
 {
+	chain();
 	const int t = blockIdx.x * blockDim.x + threadIdx.x;
 	if (t >= start_f[ctr->nb_dim[0] * ctr->nb_dim[1] * ctr->nb_dim[2]]) return;
 	const int i = __float_as_int(fp[t].w);
@@ -2790,10 +2829,11 @@ __device__ __forceinline__ bool sc_start_normal(float4 xi, float4 xj, float4 qi,
 // eight resident blocks per SM: 0.58 -> 0.50 ms per frame at 1M (the same bound made
 // the collider projection slower: 0.75 -> 0.83)
 __global__ void __launch_bounds__(kBlock, 8) k_sc_solve(int n, const StepParams* __restrict__ P,
-	const float4* __restrict__ pos, const float4* __restrict__ pos_start, const float4* __restrict__ rest,
-	const int* __restrict__ contacts, const int* __restrict__ counts, const DevCounters* __restrict__ ctr,
+	const float4* pos, const float4* pos_start, const float4* __restrict__ rest,
+	const int* contacts, const int* counts, const DevCounters* ctr,
 	float4* __restrict__ dp_out, float4* __restrict__ dp_cross)
 {
+	chain();
 	const int i = blockIdx.x * blockDim.x + threadIdx.x;
 	if (i >= n) return;
 	if (ctr->sc_contacts == 0u) return;

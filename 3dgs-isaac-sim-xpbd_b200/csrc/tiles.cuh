@@ -456,7 +456,7 @@ __device__ __forceinline__ void vt_sums(unsigned char* __restrict__ slab, const 
 // and 1 from the product, then the mean, clamp and under-relaxation per node as in the list
 // form (gather_group_lane), one thread per row.  An absent record gives zeros.  slab is free
 // again after the block's next barrier.
-template <bool NC>
+template <bool CHAIN>
 __device__ __forceinline__ void tile_gather(unsigned char* __restrict__ slab, unsigned int (&part)[2][kVtThreads / 32],
 	int n, const StepParams* __restrict__ P, const float4* __restrict__ pin, float4* __restrict__ pout,
 	const VolTile* __restrict__ tile, const int* __restrict__ rows, const unsigned int* __restrict__ pool,
@@ -483,8 +483,15 @@ __device__ __forceinline__ void tile_gather(unsigned char* __restrict__ slab, un
 		int* row_bounds = reinterpret_cast<int*>(row_pos + kVtRows);
 		float* row_len = reinterpret_cast<float*>(row_bounds + 2 * kVtRows);
 		const int row = tx < nrows ? __ldg(rows + row0 + tx) : -1;
-		const float4 m0 = ldv<NC>(pin, __ldg(&tile->mid[0])), m1 = ldv<NC>(pin, __ldg(&tile->mid[1])),
-			m2 = ldv<NC>(pin, __ldg(&tile->mid[2]));
+		if (row >= 0) {   // the row's own data, for the end
+			vt_copy4(row_bounds + 2 * tx, roff + row);
+			vt_copy4(row_bounds + 2 * tx + 1, roff + row + 1);
+			vt_copy4(row_len + tx, rest_len + row);
+		}
+		else if (tx < kVtRows) row_bounds[2 * tx] = row_bounds[2 * tx + 1] = 0;
+		const int i0 = __ldg(&tile->mid[0]), i1 = __ldg(&tile->mid[1]), i2 = __ldg(&tile->mid[2]);
+		if (CHAIN) chain_wait();   // up to here what the upload wrote
+		const float4 m0 = ldv<false>(pin, i0), m1 = ldv<false>(pin, i1), m2 = ldv<false>(pin, i2);
 		float v[4][9];
 		unsigned int valid;
 		const float3 o = vt_middle(m0, m1, m2);
@@ -497,7 +504,7 @@ __device__ __forceinline__ void tile_gather(unsigned char* __restrict__ slab, un
 				a[k] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 				b[k] = make_float4(0.0f, 0.0f, CUDART_NAN_F, 0.0f);
 				z[k] = 0.0f;
-				if (jj[k] >= 0) { ld_rec<NC>(rec, jj[k], a[k], b[k]); z[k] = ldv<NC>(recz, jj[k]); }
+				if (jj[k] >= 0) { ld_rec<false>(rec, jj[k], a[k], b[k]); z[k] = ldv<false>(recz, jj[k]); }
 			}
 			valid = 0u;
 #pragma unroll
@@ -528,13 +535,7 @@ __device__ __forceinline__ void tile_gather(unsigned char* __restrict__ slab, un
 			c0 -= kVtSlab;
 			j = columns(c0);
 		}
-		if (row >= 0) {   // the row's own data, for the end
-			vt_copy16(row_pos + tx, pin + row);
-			vt_copy4(row_bounds + 2 * tx, roff + row);
-			vt_copy4(row_bounds + 2 * tx + 1, roff + row + 1);
-			vt_copy4(row_len + tx, rest_len + row);
-		}
-		else if (tx < kVtRows) row_bounds[2 * tx] = row_bounds[2 * tx + 1] = 0;
+		if (row >= 0) vt_copy16(row_pos + tx, pin + row);
 		am = __reduce_max_sync(0xffffffffu, am);
 		av = __reduce_max_sync(0xffffffffu, av);
 		if ((tx & 31) == 0) { part[0][tx >> 5] = am; part[1][tx >> 5] = av; }
@@ -578,6 +579,7 @@ __device__ __forceinline__ void tile_gather(unsigned char* __restrict__ slab, un
 				vt_product(B, slab, c0, acc);
 			}
 			vt_sums(slab, acc, row_bounds, 1.0f / sm, 1.0f / sv);
+			if (CHAIN) chain_next();
 			if (row < 0) return;
 			const float4 p4 = row_pos[tx];
 			const float* sum = reinterpret_cast<const float*>(slab) + tx;
@@ -598,7 +600,7 @@ __device__ __forceinline__ void tile_gather(unsigned char* __restrict__ slab, un
 	if (lists)
 		for (int t = tx; t < 4 * kVtRows; t += kVtThreads) {
 			const int row = (t >> 2) < nrows ? __ldg(rows + row0 + (t >> 2)) : n;
-			gather_group_lane<4, NC>((long long)row * 4 + (t & 3), n, P, pin, pout, roff, ridx, rec, recz, rest_len);
+			gather_group_lane<4>((long long)row * 4 + (t & 3), n, P, pin, pout, roff, ridx, rec, recz, rest_len);
 		}
 }
 
