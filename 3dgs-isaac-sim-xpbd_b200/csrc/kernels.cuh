@@ -150,54 +150,67 @@ __device__ __forceinline__ bool inverse3x3_safe(const M3& M, M3& inv, float eps_
 }
 
 // cyclic-max float Jacobi, ascending eigenvalues, eigenvectors as glm columns
-// (jacobiEigenDecomposition3x3 + eigenDecomposition_glm, forward.cu:782-901)
-__device__ __noinline__ void eig_sym3f(const M3& Ag, float3& evals, M3& evecs)
+// (jacobiEigenDecomposition3x3 + eigenDecomposition_glm, forward.cu:782-901).  The pivot is
+// chosen per thread, so its entries and columns are picked by selects: indexed by p and q the
+// matrices would lie in local memory, whose traffic bound k_deformed_shapes (97 -> 54 us at
+// 250,000 Gaussians) and the float form of shape matching (24 -> 15 us at 61,000).
+__device__ __forceinline__ void eig_sym3f(const M3& Ag, float3& evals, M3& evecs)
 {
-	float A[3][3], V[3][3];
+	float a00 = Ag.m[0][0], a11 = Ag.m[1][1], a22 = Ag.m[2][2];
+	float a01 = Ag.m[1][0], a02 = Ag.m[2][0], a12 = Ag.m[2][1];
+	M3 V;
 #pragma unroll
 	for (int r = 0; r < 3; ++r)
 #pragma unroll
-		for (int c = 0; c < 3; ++c) { A[r][c] = Ag.m[c][r]; V[r][c] = (r == c) ? 1.0f : 0.0f; }
+		for (int c = 0; c < 3; ++c) V.m[c][r] = (r == c) ? 1.0f : 0.0f;
+#pragma unroll 1
 	for (int iter = 0; iter < 50; ++iter) {
-		int p = 0, q = 1;
-		float maxOff = fabsf(A[0][1]);
-		if (fabsf(A[0][2]) > maxOff) { p = 0; q = 2; maxOff = fabsf(A[0][2]); }
-		if (fabsf(A[1][2]) > maxOff) { p = 1; q = 2; maxOff = fabsf(A[1][2]); }
+		// the pivot (p, q) and the third index r: p is 0 unless it is (1, 2), q is 2 unless (0, 1)
+		float maxOff = fabsf(a01);
+		bool q2 = false, p1 = false;
+		if (fabsf(a02) > maxOff) { q2 = true; maxOff = fabsf(a02); }
+		if (fabsf(a12) > maxOff) { q2 = p1 = true; maxOff = fabsf(a12); }
 		if (maxOff < 1e-6f) break;
-		const float app = A[p][p], aqq = A[q][q], apq = A[p][q];
+		const float app = p1 ? a11 : a00, aqq = q2 ? a22 : a11;
+		const float apq = p1 ? a12 : q2 ? a02 : a01;
+		const float arp = p1 ? a01 : q2 ? a01 : a02, arq = p1 ? a02 : a12;
 		const float phi = 0.5f * (aqq - app) / (apq + 1e-20f);
-		const float t = (phi >= 0.0f) ? (1.0f / (phi + sqrtf(1.0f + phi * phi))) : (1.0f / (phi - sqrtf(1.0f + phi * phi)));
+		const float t = 1.0f / (phi >= 0.0f ? phi + sqrtf(1.0f + phi * phi) : phi - sqrtf(1.0f + phi * phi));
 		const float c = 1.0f / sqrtf(1.0f + t * t);
 		const float s = t * c;
-		A[p][p] = app - t * apq;
-		A[q][q] = aqq + t * apq;
-		A[p][q] = A[q][p] = 0.0f;
-		const int r = 3 - p - q;
-		const float arp = A[r][p], arq = A[r][q];
-		A[r][p] = A[p][r] = c * arp - s * arq;
-		A[r][q] = A[q][r] = c * arq + s * arp;
+		const float npp = app - t * apq, nqq = aqq + t * apq;
+		const float nrp = c * arp - s * arq, nrq = c * arq + s * arp;
+		a00 = p1 ? a00 : npp;
+		a11 = p1 ? npp : q2 ? a11 : nqq;
+		a22 = q2 ? nqq : a22;
+		a01 = p1 ? nrp : q2 ? nrp : 0.0f;
+		a02 = p1 ? nrq : q2 ? 0.0f : nrp;
+		a12 = p1 ? 0.0f : nrq;
 #pragma unroll
 		for (int rr = 0; rr < 3; ++rr) {
-			const float vrp = V[rr][p], vrq = V[rr][q];
-			V[rr][p] = c * vrp - s * vrq;
-			V[rr][q] = s * vrp + c * vrq;
+			const float vrp = p1 ? V.m[1][rr] : V.m[0][rr], vrq = q2 ? V.m[2][rr] : V.m[1][rr];
+			const float np = c * vrp - s * vrq, nq = s * vrp + c * vrq;
+			V.m[0][rr] = p1 ? V.m[0][rr] : np;
+			V.m[1][rr] = p1 ? np : q2 ? V.m[1][rr] : nq;
+			V.m[2][rr] = q2 ? nq : V.m[2][rr];
 		}
 	}
-	float ev[3] = { A[0][0], A[1][1], A[2][2] };
+	float ev[3] = { a00, a11, a22 };
 #pragma unroll
 	for (int i = 0; i < 2; ++i)
 #pragma unroll
-		for (int j = i + 1; j < 3; ++j)
-			if (ev[i] > ev[j]) {
-				const float te = ev[i]; ev[i] = ev[j]; ev[j] = te;
+		for (int j = i + 1; j < 3; ++j) {
+			const bool swap = ev[i] > ev[j];
+			const float lo = swap ? ev[j] : ev[i], hi = swap ? ev[i] : ev[j];
+			ev[i] = lo; ev[j] = hi;
 #pragma unroll
-				for (int rr = 0; rr < 3; ++rr) { const float tv = V[rr][i]; V[rr][i] = V[rr][j]; V[rr][j] = tv; }
+			for (int rr = 0; rr < 3; ++rr) {
+				const float vi = swap ? V.m[j][rr] : V.m[i][rr], vj = swap ? V.m[i][rr] : V.m[j][rr];
+				V.m[i][rr] = vi; V.m[j][rr] = vj;
 			}
+		}
 	evals = make_float3(ev[0], ev[1], ev[2]);
-#pragma unroll
-	for (int c = 0; c < 3; ++c)
-#pragma unroll
-		for (int rr = 0; rr < 3; ++rr) evecs.m[c][rr] = V[rr][c];
+	evecs = V;
 }
 
 // Sigma = s * SigmaHat, s = trace/3 (forward.cu:7666-7676)
@@ -1759,7 +1772,7 @@ __device__ __noinline__ bool shape_rotation_cold(const M3& A, M3& Rout, float4& 
 	return true;
 }
 
-__device__ __noinline__ bool shape_rotation_float(const M3& A, M3& Rout)
+__device__ __forceinline__ bool shape_rotation_float(const M3& A, M3& Rout)
 {
 	const M3 AtA = m3_mul(m3_t(A), A);
 	float3 S2;
@@ -3094,18 +3107,23 @@ __global__ void __launch_bounds__(kBlock) k_jstats(int n, const float4* __restri
 
 // ---------------------------------------------------------------------------
 // deformed Gaussian shapes (deformedShapeKernel, forward.cu:13063-13225; robust
-// F estimate forward.cu:450) with the FP64 Jacobi of symEig3Double (13022-13060)
+// F estimate forward.cu:450) with the FP64 Jacobi of symEig3Double (13022-13060).
+// Bound by latency of the neighbours' records and of the two iterations: the matrices stay in
+// registers, a warp's neighbour indices come through shared memory (as in k_shape_match) and
+// two neighbours' records are in flight.  Two blocks per SM; three (80 registers) and four
+// (spills) are slower.  Measured (us per launch): 250,000 Gaussians 97 -> 54.
 // ---------------------------------------------------------------------------
 // Eigen-decomposition of a symmetric 3x3 matrix in FP64 by cyclic Jacobi sweeps over the
 // pivots (0,1), (0,2), (1,2) (symEig3Double's order and stop: off-diagonal mass below
 // 1e-15 of the diagonal's, at most 32 sweeps), each rotation the one shape matching uses
 // (jacobi_rotate_d).  Columns of V: eigenvectors; ev: eigenvalues in diagonal order.
-__device__ __noinline__ void sym_eig3_double(double (&a)[3][3], double (&ev)[3], double (&V)[3][3])
+__device__ __forceinline__ void sym_eig3_double(double (&a)[3][3], double (&ev)[3], double (&V)[3][3])
 {
 #pragma unroll
 	for (int r = 0; r < 3; ++r)
 #pragma unroll
 		for (int c = 0; c < 3; ++c) V[r][c] = (r == c) ? 1.0 : 0.0;
+#pragma unroll 1
 	for (int sweep = 0; sweep < 32; ++sweep) {
 		const double off = fabs(a[0][1]) + fabs(a[0][2]) + fabs(a[1][2]);
 		const double diag = fabs(a[0][0]) + fabs(a[1][1]) + fabs(a[2][2]);
@@ -3117,13 +3135,23 @@ __device__ __noinline__ void sym_eig3_double(double (&a)[3][3], double (&ev)[3],
 	ev[0] = a[0][0]; ev[1] = a[1][1]; ev[2] = a[2][2];
 }
 
-__global__ void __launch_bounds__(kBlock) k_deformed_shapes(int n, const float4* __restrict__ rest,
+__global__ void __launch_bounds__(kBlock, 2) k_deformed_shapes(int n, const float4* __restrict__ rest,
 	const float4* __restrict__ cur, const int* __restrict__ off, const int* __restrict__ nbr,
 	const float* __restrict__ scales, const float* __restrict__ rots, float deform_eps, float* __restrict__ out_scale,
 	float* __restrict__ out_quat, DevCounters* __restrict__ ctr, const int* __restrict__ perm)
 {
+	__shared__ int s_nbr[kBlock / 32][kShapeWindow];
 	const int i = blockIdx.x * blockDim.x + threadIdx.x;
+	const int row0 = i & ~31;
+	if (row0 >= n) return;
+	int* window = s_nbr[threadIdx.x >> 5];
+	const int begin = __ldg(off + row0), end = __ldg(off + min(row0 + 32, n));
+	const bool held = end - begin <= kShapeWindow;
+	if (held)
+		for (int e = begin + (threadIdx.x & 31); e < end; e += 32) window[e - begin] = __ldg(nbr + e);
+	__syncwarp();
 	if (i >= n) return;
+	auto at = [&](int e) { return held ? window[e - begin] : __ldg(nbr + e); };
 	const int o = perm ? perm[i] : i;   // output slot in the caller's order
 	const float3 s0 = make_float3(scales[3 * i], scales[3 * i + 1], scales[3 * i + 2]);
 	const float4 q0 = make_float4(rots[4 * i], rots[4 * i + 1], rots[4 * i + 2], rots[4 * i + 3]);
@@ -3138,14 +3166,20 @@ __global__ void __launch_bounds__(kBlock) k_deformed_shapes(int n, const float4*
 		M3 PPt, QPt;
 		m3_zero(PPt);
 		m3_zero(QPt);
-		for (int k = 0; k < kn; ++k) {
-			const int j = nbr[e0 + k];
-			if (j < 0 || j >= n) continue;
-			const float4 rj = rest[j], cj = cur[j];
+		auto add = [&](float4 rj, float4 cj) {
 			const float3 p = make_float3(rj.x - x0.x, rj.y - x0.y, rj.z - x0.z);
 			const float3 q = make_float3(cj.x - x.x, cj.y - x.y, cj.z - x.z);
 			m3_add_outer(PPt, p, p);
 			m3_add_outer(QPt, q, p);
+		};
+		for (int k = 0; k < kn; k += 2) {   // two neighbours' loads in flight
+			const int j0 = at(e0 + k), j1 = k + 1 < kn ? at(e0 + k + 1) : -1;
+			const bool ok0 = j0 >= 0 && j0 < n, ok1 = j1 >= 0 && j1 < n;
+			float4 r0 = make_float4(0.0f, 0.0f, 0.0f, 0.0f), r1 = r0, c0 = r0, c1 = r0;
+			if (ok0) { r0 = ld4(rest, j0); c0 = ld4(cur, j0); }
+			if (ok1) { r1 = ld4(rest, j1); c1 = ld4(cur, j1); }
+			if (ok0) add(r0, c0);
+			if (ok1) add(r1, c1);
 		}
 		const float tr_p = PPt.m[0][0] + PPt.m[1][1] + PPt.m[2][2];
 		const float alpha = (tr_p > 0.0f) ? (tr_p * 1e-4f) : 1e-6f;
