@@ -100,6 +100,7 @@ struct DBuf {
 		n = 0;
 	}
 	size_t bytes() const { return sizeof(T) * n; }
+	void swap(DBuf& o) { std::swap(p, o.p); std::swap(n, o.n); }
 };
 
 // Rows in chunks of 256, each chunk sorted by list length (longest first): the groups of a
@@ -189,14 +190,12 @@ public:
 	// ---- device state ----
 	DBuf<float4> pos_curr, pos_next, pos_tmp, vel, pos_rest, shape_rest;
 	DBuf<float4> shape_q;    // per Gaussian: eigenvector frame of its last FP64 polar decomposition
-	// ChainMail: (arrival time, density), sweep flags / marks / work list / scratch, seeds
-	DBuf<float2> cm_td;
-	DBuf<unsigned char> cm_flag;
-	DBuf<unsigned int> cm_mark;
-	DBuf<int> cm_work, cm_seed_idx;
-	DBuf<float4> cm_spos;
-	DBuf<float> cm_stime, cm_seed_delta, cm_time_out;
-	DBuf<dev::CmState> cm_state;
+	// ChainMail: (arrival time, density) and the mask of changed Gaussians, each with the copy
+	// that a sweep writes; whether the last sweeps changed anything; seeds
+	DBuf<float2> cm_td, cm_td_next;
+	DBuf<unsigned int> cm_mask, cm_mask_next;
+	DBuf<int> cm_changed, cm_seed_idx;
+	DBuf<float> cm_seed_delta, cm_time_out;
 	// object mode: rest offsets q (FP64, internal order), per-object rest centroid, sum q,
 	// count, previous centroid, fit parameters, centroid move, block partials, fit weights,
 	// boxes; self-collision active set, cross-object corrections and their frame sums
@@ -476,8 +475,8 @@ public:
 	{
 		pos_curr.release(); pos_next.release(); pos_tmp.release(); vel.release(); pos_rest.release();
 		shape_rest.release(); shape_q.release();
-		cm_td.release(); cm_flag.release(); cm_mark.release(); cm_work.release(); cm_seed_idx.release();
-		cm_spos.release(); cm_stime.release(); cm_seed_delta.release(); cm_time_out.release(); cm_state.release();
+		cm_td.release(); cm_td_next.release(); cm_mask.release(); cm_mask_next.release(); cm_changed.release();
+		cm_seed_idx.release(); cm_seed_delta.release(); cm_time_out.release();
 		obj_q.release(); obj_shift.release(); obj_sumq.release(); obj_partial.release(); obj_c0.release();
 		obj_params.release(); obj_disp.release(); obj_w.release(); obj_boxes.release(); push_partial.release();
 		push_T.release(); obj_count.release(); sc_active.release(); sc_cross.release(); sc_accum.release();
@@ -1072,12 +1071,10 @@ public:
 		const auto dens = to_internal(in_opacity.data(), 1);
 		std::vector<float2> td(n);
 		for (int i = 0; i < n; ++i) td[i] = make_float2(1e9f, dens[i]);
-		CK(cm_td.alloc(n)); CK(cm_flag.alloc(n)); CK(cm_mark.alloc((n + 31) / 32)); CK(cm_work.alloc(n));
-		CK(cm_spos.alloc(n)); CK(cm_stime.alloc(n)); CK(cm_time_out.alloc(n)); CK(cm_state.alloc(1));
+		CK(cm_td_next.alloc(n)); CK(cm_mask.alloc((n + 31) / 32)); CK(cm_mask_next.alloc((n + 31) / 32));
+		CK(cm_time_out.alloc(n)); CK(cm_changed.alloc(4)); CK(cm_td.alloc(n));
 		CK(cudaMemcpyAsync(cm_td.p, td.data(), sizeof(float2) * n, cudaMemcpyHostToDevice, stream));
-		CK(cudaMemsetAsync(cm_flag.p, 0, cm_flag.bytes(), stream));
-		CK(cudaMemsetAsync(cm_mark.p, 0, cm_mark.bytes(), stream));
-		CK(cudaMemsetAsync(cm_state.p, 0, cm_state.bytes(), stream));
+		CK(cudaMemsetAsync(cm_mask.p, 0, cm_mask.bytes(), stream));
 		return sync();
 	}
 
@@ -1097,8 +1094,7 @@ public:
 		if ((int)cm_seed_idx.n < count) { CK(cm_seed_idx.alloc(count)); CK(cm_seed_delta.alloc(3 * (size_t)count)); }
 		CK(cudaMemcpyAsync(cm_seed_idx.p, ii.data(), sizeof(int) * count, cudaMemcpyHostToDevice, stream));
 		CK(cudaMemcpyAsync(cm_seed_delta.p, delta, sizeof(float) * 3 * count, cudaMemcpyHostToDevice, stream));
-		dev::k_cm_seed<<<1, 1, 0, stream>>>(count, cm_seed_idx.p, cm_seed_delta.p, pos_curr.p, cm_td.p, cm_flag.p,
-			cm_state.p);
+		dev::k_cm_seed<<<1, 32, 0, stream>>>(count, cm_seed_idx.p, cm_seed_delta.p, pos_curr.p, cm_td.p, cm_mask.p);
 		CK(cudaGetLastError());
 		if (cm_publish(nullptr)) return -1;
 		return sync();
@@ -1110,20 +1106,18 @@ public:
 	{
 		if (ensure_chainmail()) return -1;
 		const dev::CmMaterial M = S.cm;
-		const dim3 B(kBlock);
-		const dim3 G = blocks_for(n);
-		const dim3 GS(std::min<unsigned>(G.x, 148u * 8u));   // grid-stride kernels
-		for (int it = 0; it < prop_iters; ++it) {
-			dev::k_cm_begin<<<1, 1, 0, stream>>>(n, S.cm_frontier ? n / 4 : -1, cm_state.p);
-			dev::k_cm_expand<<<GS, B, 0, stream>>>(n, off.p, nbr.p, cm_flag.p, cm_mark.p, cm_work.p, cm_state.p);
-			dev::k_cm_sweep<<<GS, B, 0, stream>>>(n, pos_curr.p, cm_td.p, off.p, nbr.p, ndist.p, nstiff.p, cm_work.p,
-				cm_state.p, M, strength, cm_spos.p, cm_stime.p);
-			dev::k_cm_commit<<<GS, B, 0, stream>>>(n, pos_curr.p, cm_td.p, cm_work.p, cm_spos.p, cm_stime.p, cm_flag.p,
-				cm_mark.p, cm_state.p);
-			launches += 4;
-		}
+		const dim3 B(dev::kCmWarps * 32), G = blocks_for(n, dev::kCmWarps * 32);
 		float4* a = pos_curr.p;
 		float4* b = pos_tmp.p;
+		if (prop_iters) CK(cudaMemsetAsync(cm_changed.p, 0, cm_changed.bytes(), stream));
+		for (int it = 0; it < prop_iters; ++it) {
+			dev::k_cm_sweep<<<G, B, 0, stream>>>(n, it, S.cm_frontier ? 0 : 1, a, cm_td.p, b, cm_td_next.p, cm_mask.p,
+				cm_mask_next.p, cm_changed.p, off.p, nbr.p, ndist.p, nstiff.p, M, strength);
+			++launches;
+			std::swap(a, b);
+			cm_td.swap(cm_td_next);
+			cm_mask.swap(cm_mask_next);
+		}
 		for (int it = 0; it <= relax_iters; ++it) {
 			dev::k_cm_relax<<<G, B, 0, stream>>>(n, a, b, cm_td.p, off.p, nbr.p, ndist.p, nstiff.p, M, stiffness, damping);
 			++launches;
