@@ -2358,7 +2358,7 @@ static int render_bin(Engine& E, long long m, int tiles_x, int tiles)
 	CK(cub::DeviceRadixSort::SortPairs(nullptr, t3b, tk, tks, R.val.p, R.val_s.p, (int)m, 0, bits, st));
 	if (R.temp.n < t3b) CK(R.temp.alloc(t3b));
 	CK(cub::DeviceRadixSort::SortPairs(R.temp.p, t3b, tk, tks, R.val.p, R.val_s.p, (int)m, 0, bits, st));
-	dev::k_splat_ranges<Key><<<Engine::blocks_for(tiles), kBlock, 0, st>>>(tiles, (int)m, tks, R.ranges.p);
+	dev::k_splat_ranges<Key><<<Engine::blocks_for((m * (long long)sizeof(Key) + 15) / 16), kBlock, 0, st>>>((int)m, tks, R.ranges.p);
 	CK(cudaGetLastError());
 	E.launches += 2;
 	return 0;
@@ -2485,16 +2485,14 @@ static long long render_frame(Engine& E, const float* view, const float* proj, c
 		F.fl_inv_fade2 = 1.0f / fmaxf(R.floor_fade * R.floor_fade, 1e-12f);
 	}
 	// 1. project every Gaussian
+	CK(cudaMemsetAsync(R.d_total.p, 0, sizeof(unsigned long long), st));
 	dev::k_splat_prepare<<<Engine::blocks_for(n), kBlock, 0, st>>>(n, F, E.pos_out3.p, sc, q, R.opacity.p,
-		R.colors.p, R.xy.p, R.conic.p, R.rgb.p, R.dkey.p, R.radii.p, R.rect.p, R.touched.p);
+		R.colors.p, R.xy.p, R.conic.p, R.rgb.p, R.dkey.p, R.radii.p, R.rect.p, R.touched.p, R.d_total.p);
 	CK(cudaGetLastError());
 	seg_end(ST_RENDER_PREPARE, seg);
 	seg = seg_begin();
 	// 2. the pair count goes to the host while the GPU sorts by depth and scans the
 	// tile counts in that order; the host waits for it only before the pair stage
-	CK(cudaMemsetAsync(R.d_total.p, 0, sizeof(unsigned long long), st));
-	dev::k_splat_total<<<Engine::blocks_for(n), kBlock, 0, st>>>(n, R.touched.p, R.d_total.p);
-	CK(cudaGetLastError());
 	CK(cudaMemcpyAsync(R.h_total, R.d_total.p, sizeof(long long), cudaMemcpyDeviceToHost, st));
 	if (!R.ev_total) CK(cudaEventCreateWithFlags(&R.ev_total, cudaEventDisableTiming));
 	CK(cudaEventRecord(R.ev_total, st));
@@ -2508,7 +2506,7 @@ static long long render_frame(Engine& E, const float* view, const float* proj, c
 	CK(cudaGetLastError());
 	CK(cudaMemsetAsync(R.offs.p, 0, sizeof(long long), st));
 	CK(cub::DeviceScan::InclusiveSum(R.temp.p, t2b, R.cnt.p, R.offs.p + 1, n, st));
-	E.launches += 3;
+	E.launches += 2;
 	CK(cudaEventSynchronize(R.ev_total));
 	const long long m = *R.h_total;
 	if (m < 0 || m > INT_MAX) return fail("xpbd_b200_render: %lld tile pairs (limit %d)", m, INT_MAX);
