@@ -1610,6 +1610,11 @@ public:
 		float4* pin = pos_next.p;
 		float4* pout = pos_tmp.p;
 		const bool dgs = dist_gs_on(), vgs = vol_gs_on();
+		// eight rows a warp while all the warps fit on the chip at once (148 SMs of nine blocks),
+		// where a launch is one warp's chain of loads.  A frame with 8 and with 32 rows a warp:
+		// 2,000 Gaussians 1.79 and 1.88 ms, 20,000 2.08 and 2.16, 61,000 2.39 and 2.35, 200,000
+		// 6.31 and 6.02
+		const bool few_rows = N <= 148 * 9 * dev::kDistWarps * 8;
 		const bool project = S.kin_count > 0 || !S.kin_ext.empty() || S.ground_on || sc || press_active;
 		for (int it = 0; it < S.iters; ++it) {
 			const int first = (it == 0), last = (it == S.iters - 1);
@@ -1624,10 +1629,10 @@ public:
 			}
 			else if (S.use_distance) {
 				if (N <= 1 << dev::kCodeBits)
-					launch(ST_DISTANCE, blocks_for(N, dev::kDistWarps * 32), dim3(dev::kDistWarps * 32), dev::k_distance_jacobi, N,
-						(const StepParams*)d_params, (const float4*)pin, pout, (const int*)off.p,
-						(const unsigned int*)ecode.p, (const float*)ndist.p, (const float*)nstiff.p, lam.p, first ? 0 : 1,
-						last ? 0 : 1);
+					launch(ST_DISTANCE, blocks_for(N, dev::kDistWarps * (few_rows ? 8 : 32)), dim3(dev::kDistWarps * 32),
+						few_rows ? dev::k_distance_jacobi<8> : dev::k_distance_jacobi<32>, N, (const StepParams*)d_params,
+						(const float4*)pin, pout, (const int*)off.p, (const unsigned int*)ecode.p, (const float*)ndist.p,
+						(const float*)nstiff.p, lam.p, first ? 0 : 1, last ? 0 : 1);
 				else
 					launch(ST_DISTANCE, G, B, dev::k_distance_rows, N, (const StepParams*)d_params, (const float4*)pin, pout,
 						(const int*)off.p, (const int*)nbr.p, (const float*)ndist.p, (const float*)nstiff.p, lam.p,

@@ -25,6 +25,7 @@ namespace dev {
 // kernel implies the end of all before it.  Launched without the attribute both are no-ops.
 // A chained kernel runs beside the one whose results it reads, so those results never take
 // the read-only (non-coherent) path: ldv<false>, or pointers without __restrict__.
+// k_distance_jacobi waits for the whole of its predecessor (chained it was no faster).
 // The long kernels call chain_next near their ends: the next kernel's blocks are placed where
 // there is room, and placed while an uneven kernel still fills half of the SMs they crowd the
 // other half (61,000 Gaussians, a frame: 2.80 ms unchained, 3.27 with chain_next first, 2.69
@@ -424,18 +425,19 @@ __global__ void __launch_bounds__(kBlock) k_distance_rows(int n, const StepParam
 		write_lam);
 }
 
-// A warp per 32 rows.  Their edges are one run of the CSR arrays: the lanes take them 32 at a
-// time (coalesced, every lane busy whatever the rows' degrees, the loads of five trips in
-// flight together), leave each correction in shared memory, and then every lane adds its own
-// row's in row order.  With a thread per row, loading its 8 to 18 edges two at a time, the
-// kernel was bound by the wavefronts of strided loads and, in small scenes, by the chain of
-// dependent ones.  ecode: an edge's neighbour, and its row modulo 32 in the top five bits.
-// Measured (us per launch): 1,000,000
-// Gaussians 84 -> 71, 200,000 28 -> 21, 20,000 13.6 -> 10.8, 250,000 of degree 14 52 -> 34.
+// A warp per 32 rows (in small scenes 8: few_rows in the step).  Their edges are one run of the
+// CSR arrays: the lanes take them 32 at a time (coalesced, every lane busy whatever the rows'
+// degrees, the loads of five trips in flight together), leave each correction in shared memory,
+// and then every lane adds its own row's in row order.  With a thread per row, loading its 8 to
+// 18 edges two at a time, the kernel was bound by the wavefronts of strided loads and, in small
+// scenes, by the chain of dependent ones.  ecode: an edge's neighbour, and its row modulo 32 in
+// the top five bits.  Measured (us per launch): 1,000,000 Gaussians 84 -> 71, 200,000 28 -> 21,
+// 20,000 13.6 -> 10.8 with 32 rows, 8.5 with 8, 250,000 of degree 14 52 -> 34.
 constexpr int kDistWarps = 4;        // warps per block
 constexpr int kDistTrips = 5;        // edges per lane in flight
 constexpr int kDistWindow = 320;     // edges per pass: two batches of trips (mean degree 9.3: one pass)
 constexpr int kCodeBits = 27;
+template <int ROWS>
 __global__ void __launch_bounds__(kDistWarps * 32) k_distance_jacobi(int n, const StepParams* __restrict__ P,
 	const float4* __restrict__ pin, float4* __restrict__ pout, const int* __restrict__ off,
 	const unsigned int* __restrict__ ecode, const float* __restrict__ ndist, const float* __restrict__ nstiff,
@@ -444,12 +446,11 @@ __global__ void __launch_bounds__(kDistWarps * 32) k_distance_jacobi(int n, cons
 	__shared__ float4 s_row[kDistWarps][32];            // the rows' positions
 	__shared__ float4 s_corr[kDistWarps][kDistWindow];  // corrections; w = 1 where the edge counts
 	const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-	const int row0 = (blockIdx.x * kDistWarps + w) * 32;
+	const int row0 = (blockIdx.x * kDistWarps + w) * ROWS;
 	if (row0 >= n) return;
-	const int row = row0 + lane;
+	const int row = lane < ROWS ? row0 + lane : n;
 	const int e0 = off[min(row, n)], e1 = off[min(row + 1, n)];
-	const int begin = __shfl_sync(0xffffffffu, e0, 0), end = __shfl_sync(0xffffffffu, e1, 31);
-	chain_wait();
+	const int begin = __shfl_sync(0xffffffffu, e0, 0), end = __shfl_sync(0xffffffffu, e1, ROWS - 1);
 	float4 p4 = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 	if (row < n) p4 = ldv<false>(pin, row);
 	s_row[w][lane] = p4;
@@ -479,7 +480,7 @@ __global__ void __launch_bounds__(kDistWarps * 32) k_distance_jacobi(int n, cons
 #pragma unroll
 			for (int t = 0; t < kDistTrips; ++t)
 				if (at + 32 * t < w1) {
-					const float4 own = s_row[w][code[t] >> kCodeBits];
+					const float4 own = s_row[w][(code[t] >> kCodeBits) & (ROWS - 1)];
 					const float wi = own.w * ims;
 					float4 out = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 					float3 c;

@@ -56,3 +56,18 @@ def test_rows_and_rotations_match_oracle(n, hubs, pose, robust):
         solver.destroy()
     assert np.isfinite(out[1]).all()
     assert H.max_err_over_diag(out[0], out[1], H.scenes.bbox_diagonal(out[1])) < H.TOL_1STEP
+
+
+@pytest.mark.parametrize("n", [9, 42624, 42625])
+def test_rows_per_warp_match_oracle(n):
+    """Distance on both sides of the limit where a warp takes 8 rows instead of 32 (148 SMs x 9
+    blocks x 4 warps x 8 rows); the one-step tolerance."""
+    sc = _hub_scene(n, (0,) if n > 1000 else ())
+    out = []
+    for solver in (H.b200(), H.oracle()):
+        scen = H.scenes.Scenario(sc, [], iters=2, volume=False, shape=False)
+        scen.setup(solver)
+        solver.step()
+        out.append(solver.positions())
+        solver.destroy()
+    assert H.max_err_over_diag(out[0], out[1], H.scenes.bbox_diagonal(out[1])) < H.TOL_1STEP
