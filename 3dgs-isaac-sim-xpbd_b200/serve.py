@@ -34,9 +34,10 @@ BYTES_PER_GAUSSIAN = 3200   # a session engine of its own: state, graph, cluster
 # arena bytes per row (Gaussian): 7 float4 state arrays, caller-order positions, order,
 # object id, multiplier, rest volume terms, material, cluster record, saved inverse
 # mass, three CSR row starts (212 B), the volume gather's tile rows, list rows and tiles (10 B)
-# and tile words (at most the reverse entries' size); per directed edge 16 B, per member and
-# reverse entry 4 B
-ARENA_ROW_BYTES = 222 + 4 * 68
+# and tile words (at most the reverse entries' size), the member lists' group and padding to
+# groups of 16 (64 B) and the edge codes (4 B per directed edge); per directed edge 16 B more,
+# per member and reverse entry 4 B
+ARENA_ROW_BYTES = 222 + 4 * 68 + 64 + 4 * 12
 ARENA_EDGES, ARENA_MEMBERS, ARENA_REV = 12, 66, 68      # capacity per row (8-NN graph, 64-member clusters)
 
 
