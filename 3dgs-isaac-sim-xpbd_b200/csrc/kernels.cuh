@@ -154,7 +154,11 @@ __device__ __forceinline__ bool inverse3x3_safe(const M3& M, M3& inv, float eps_
 // (jacobiEigenDecomposition3x3 + eigenDecomposition_glm, forward.cu:782-901).  The pivot is
 // chosen per thread, so its entries and columns are picked by selects: indexed by p and q the
 // matrices would lie in local memory, whose traffic bound k_deformed_shapes (97 -> 54 us at
-// 250,000 Gaussians) and the float form of shape matching (24 -> 15 us at 61,000).
+// 250,000 Gaussians) and the float form of shape matching (24 -> 15 us at 61,000).  Every
+// rounding is written out: the compiler may fuse c x - s y and c x + s y either way, a last bit
+// here decides the order of two nearly equal axes of a deformed Gaussian, and callers keep
+// those.  These are the roundings of the indexed form (nrq's other fusion gives other values
+// for a Gaussian in eight).
 __device__ __forceinline__ void eig_sym3f(const M3& Ag, float3& evals, M3& evecs)
 {
 	float a00 = Ag.m[0][0], a11 = Ag.m[1][1], a22 = Ag.m[2][2];
@@ -175,12 +179,13 @@ __device__ __forceinline__ void eig_sym3f(const M3& Ag, float3& evals, M3& evecs
 		const float app = p1 ? a11 : a00, aqq = q2 ? a22 : a11;
 		const float apq = p1 ? a12 : q2 ? a02 : a01;
 		const float arp = p1 ? a01 : q2 ? a01 : a02, arq = p1 ? a02 : a12;
-		const float phi = 0.5f * (aqq - app) / (apq + 1e-20f);
-		const float t = 1.0f / (phi >= 0.0f ? phi + sqrtf(1.0f + phi * phi) : phi - sqrtf(1.0f + phi * phi));
-		const float c = 1.0f / sqrtf(1.0f + t * t);
-		const float s = t * c;
-		const float npp = app - t * apq, nqq = aqq + t * apq;
-		const float nrp = c * arp - s * arq, nrq = c * arq + s * arp;
+		const float phi = __fdiv_rn(__fmul_rn(0.5f, __fsub_rn(aqq, app)), __fadd_rn(apq, 1e-20f));
+		const float root = __fsqrt_rn(__fmaf_rn(phi, phi, 1.0f));
+		const float t = __frcp_rn(phi >= 0.0f ? __fadd_rn(phi, root) : __fsub_rn(phi, root));
+		const float c = __frcp_rn(__fsqrt_rn(__fmaf_rn(t, t, 1.0f)));
+		const float s = __fmul_rn(t, c);
+		const float npp = __fmaf_rn(-t, apq, app), nqq = __fmaf_rn(t, apq, aqq);
+		const float nrp = __fmaf_rn(c, arp, -__fmul_rn(s, arq)), nrq = __fmaf_rn(s, arp, __fmul_rn(c, arq));
 		a00 = p1 ? a00 : npp;
 		a11 = p1 ? npp : q2 ? a11 : nqq;
 		a22 = q2 ? nqq : a22;
@@ -190,7 +195,7 @@ __device__ __forceinline__ void eig_sym3f(const M3& Ag, float3& evals, M3& evecs
 #pragma unroll
 		for (int rr = 0; rr < 3; ++rr) {
 			const float vrp = p1 ? V.m[1][rr] : V.m[0][rr], vrq = q2 ? V.m[2][rr] : V.m[1][rr];
-			const float np = c * vrp - s * vrq, nq = s * vrp + c * vrq;
+			const float np = __fmaf_rn(c, vrp, -__fmul_rn(s, vrq)), nq = __fmaf_rn(s, vrp, __fmul_rn(c, vrq));
 			V.m[0][rr] = p1 ? V.m[0][rr] : np;
 			V.m[1][rr] = p1 ? np : q2 ? V.m[1][rr] : nq;
 			V.m[2][rr] = q2 ? nq : V.m[2][rr];
