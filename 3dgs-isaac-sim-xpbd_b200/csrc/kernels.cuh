@@ -1712,8 +1712,11 @@ __device__ __forceinline__ bool shape_rotation_newton(const M3& A, M3& Rout, flo
 		C00 = H11 * H22 - H12 * H12; C01 = H02 * H12 - H01 * H22; C02 = H01 * H12 - H02 * H11;
 		C22 = H00 * H11 - H01 * H01;
 		const float det = H00 * C00 + H01 * C01 + H02 * C02, tr = H00 + H11 + H22;
-		// positive definite, and by 4 det > 1e-3 tr^3 its smallest eigenvalue above 1e-3 tr
-		if (!(H00 > 0.0f && C22 > 0.0f && 4.0f * det > 1e-3f * tr * tr * tr)) return false;
+		// positive definite, and by 4 det > 1e-3 tr^3 its smallest eigenvalue above 1e-3 tr.  The
+		// trace decides between the maximum and a saddle half a turn away: there the matrix of a
+		// nearly isotropic A is two small numbers and -2/3 |A|, its first two minors can be
+		// positive and the cube is then the smaller side
+		if (!(H00 > 0.0f && C22 > 0.0f && tr > 0.0f && 4.0f * det > 1e-3f * tr * tr * tr)) return false;
 		C11 = H00 * H22 - H02 * H02; C12 = H01 * H02 - H00 * H12;
 		const float inv = 1.0f / det;
 		C00 *= inv; C01 *= inv; C02 *= inv; C11 *= inv; C12 *= inv; C22 *= inv;
