@@ -1684,8 +1684,11 @@ __device__ __forceinline__ void quat_turn(T (&q)[4], T x, T y, T z)
 //   (tr B I - (B + B^T) / 2) w = axial(B - B^T),   R <- R exp([w]),
 // which converges cubically (the third-order term vanishes where B is symmetric).  FP32 steps
 // take it to FP32 rounding; then the residual axial(B - B^T) is formed in FP64 and corrected
-// with the FP32 matrix until the correction is below 3e-7, which leaves an error of 1e-12 or
-// less, the Jacobi iteration's own stop.  One step of each where the FP64 Jacobi run takes
+// with the FP32 matrix until the correction is below 3e-7.  The matrix is the one where the
+// FP32 steps end, right to its own rounding, so what is left of a correction is 1e-6 of it over
+// the matrix's condition: 7e-14 for singular values within a factor of five of one another,
+// 4e-12 for needles of 1 : 1000 (worst of 200,000 each against an FP64 SVD; with the matrix
+// from before the last step 3e-10 and 3e-8).  One step of each where the FP64 Jacobi run takes
 // AtA, two conjugations, one or two rotations and U V^T: about 80 FP64 operations for 350.
 // The matrix is positive definite only around the maximum, so a step that finds it is not
 // well so (its smallest eigenvalue, the sum of the two smallest singular values, under a
@@ -1699,8 +1702,8 @@ __device__ __forceinline__ bool shape_rotation_newton(const M3& A, M3& Rout, flo
 		if (!(n2 > 0.5f && n2 < 2.0f)) { q[0] = 1.0f; q[1] = q[2] = q[3] = 0.0f; }
 	}
 	float C00, C01, C02, C11, C12, C22;   // inverse of the Newton matrix
-	float w2 = 1.0f;
-	for (int it = 0; it < 5; ++it) {
+	bool near = false;
+	for (int it = 0;; ++it) {   // up to five steps, then the matrix where they end
 		float R[3][3], B[3][3];
 		quat_matrix(q, R);
 #pragma unroll
@@ -1720,18 +1723,19 @@ __device__ __forceinline__ bool shape_rotation_newton(const M3& A, M3& Rout, flo
 		C11 = H00 * H22 - H02 * H02; C12 = H01 * H02 - H00 * H12;
 		const float inv = 1.0f / det;
 		C00 *= inv; C01 *= inv; C02 *= inv; C11 *= inv; C12 *= inv; C22 *= inv;
+		if (near) break;
+		if (it == 5) return false;
 		const float ax = B[2][1] - B[1][2], ay = B[0][2] - B[2][0], az = B[1][0] - B[0][1];
 		const float x = C00 * ax + C01 * ay + C02 * az, y = C01 * ax + C11 * ay + C12 * az,
 			z = C02 * ax + C12 * ay + C22 * az;
-		w2 = x * x + y * y + z * z;
+		const float w2 = x * x + y * y + z * z;
 		if (!(w2 < 0.25f)) return false;
 		quat_turn(q, x, y, z);
 		const float s = 1.5f - 0.5f * (q[0] * q[0] + q[1] * q[1] + q[2] * q[2] + q[3] * q[3]);   // to unit length, |w| small
 #pragma unroll
 		for (int k = 0; k < 4; ++k) q[k] *= s;
-		if (w2 < 1e-5f) break;
+		near = w2 < 1e-5f;
 	}
-	if (!(w2 < 1e-5f)) return false;
 	double d[4] = { q[0], q[1], q[2], q[3] }, R[3][3];
 	double m2 = 1.0;
 	for (int it = 0; it < 4; ++it) {
