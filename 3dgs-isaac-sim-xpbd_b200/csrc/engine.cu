@@ -1330,9 +1330,11 @@ public:
 	bool dist_gs_on() const { return S.use_distance && S.dist_gs && coloring_built && !coloring.edge.empty(); }
 	bool vol_gs_on() const { return S.use_volume && S.vol_gs && clusters.gs_color_off.size() > 1; }
 
+	// what a captured step depends on; the lanes as set, too: 4 and automatic are different kernels
 	std::vector<long long> topology_key() const
 	{
 		return { (long long)generation, S.iters, S.use_distance, dist_gs_on(), S.use_volume, vol_gs_on(), vol_lanes(), gather_lanes(),
+			S.lanes_a, S.lanes_b,
 			S.use_shape, S.shape_robust, selfcol_on(), S.kin_count > 0 || S.ground_on || selfcol_on() || press_active, S.jstats,
 			(long long)S.kin_ext.empty(), (long long)(size_t)d_kin_ext.p,
 			(long long)coloring.color_off.size(), (long long)clusters.gs_color_off.size(), (long long)sc_table,

@@ -1,0 +1,53 @@
+"""The switches between the step's forms: which kernels a step runs, and what comes out."""
+import ctypes
+
+import numpy as np
+import pytest
+
+import helpers as H
+
+pytestmark = pytest.mark.gpu
+
+ITERS = 3
+
+
+def _lanes(solver, solve, gather):
+    solver.lib.xpbd_b200_set_volume_lanes.argtypes = [ctypes.c_int] * 2
+    solver.lib.xpbd_b200_set_volume_lanes(solve, gather)
+
+
+def _tuning(solver):
+    t = np.zeros(7, np.float32)
+    solver.lib.xpbd_b200_tuning.argtypes = [ctypes.c_void_p]
+    solver.lib.xpbd_b200_tuning(t.ctypes.data)
+    return t
+
+
+@pytest.fixture
+def lib():
+    solver = H.b200()
+    yield solver
+    _lanes(solver, 0, 0)
+    solver.destroy()
+
+
+def _mixed(solver):
+    """Rows in tiles and, in a small component, rows in the list form."""
+    scene = H.scenes.merge_scenes([H.scenes.make_scene(300, 1), H.scenes.make_scene(40, 2, centre=(4.0, 0.0, 0.0))])
+    H.scenes.Scenario(scene, [], iters=ITERS, shape=False).setup(solver)
+    return scene
+
+
+def test_lanes_set_after_a_step_take_effect(lib):
+    """Automatic: a launch for the tiles and one for the lists; four lanes: the lists alone."""
+    _mixed(lib)
+    lib.step()
+    tiles, rows = lib.ints("gather_tiles")
+    assert tiles > 0 and rows == 40
+    both = _tuning(lib)[4]
+    _lanes(lib, 0, 4)
+    lib.step()
+    assert _tuning(lib)[4] == both - ITERS
+    _lanes(lib, 0, 0)
+    lib.step()
+    assert _tuning(lib)[4] == both
