@@ -1489,7 +1489,7 @@ public:
 	bool fused_eligible() const
 	{
 		return !selfcol_on() && !object_on() && !dist_gs_on() && !vol_gs_on() &&
-			(!S.use_volume || (vol_lanes() == 4 && S.lanes_a == 0 && gather_lanes() == 4)) && !S.use_angle && n > 0;
+			(!S.use_volume || (vol_lanes() == 4 && S.lanes_a == 0 && gather_lanes() == 4 && S.lanes_b == 0)) && !S.use_angle && n > 0;
 	}
 
 	// the sorted lists unpacked, before a step that reads them

@@ -23,11 +23,17 @@ def _tuning(solver):
     return t
 
 
+def _fused(solver, mode):
+    solver.lib.xpbd_b200_set_fused.argtypes = [ctypes.c_int]
+    solver.lib.xpbd_b200_set_fused(mode)
+
+
 @pytest.fixture
 def lib():
     solver = H.b200()
     yield solver
     _lanes(solver, 0, 0)
+    _fused(solver, 0)
     solver.destroy()
 
 
@@ -51,3 +57,14 @@ def test_lanes_set_after_a_step_take_effect(lib):
     _lanes(lib, 0, 0)
     lib.step()
     assert _tuning(lib)[4] == both
+
+
+def test_lists_asked_for_leave_the_fused_form(lib):
+    """The fused launch runs the tiles, so it does not stand in for the list form."""
+    _mixed(lib)
+    _fused(lib, 1)
+    lib.step()
+    assert _tuning(lib)[0] == 1.0
+    _lanes(lib, 0, 4)
+    lib.step()
+    assert _tuning(lib)[0] == 0.0
