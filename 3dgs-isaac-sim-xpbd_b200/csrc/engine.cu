@@ -1537,6 +1537,7 @@ public:
 	{
 		if (!fused_grid) {
 			int dev_id = 0, sms = 0, per_sm = 0;
+			if (prepare_tile_kernels()) return -1;   // the upload did so only if there was a tile to build
 			CK(cudaGetDevice(&dev_id));
 			CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev_id));
 			CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, dev::k_substep_fused, kBlock, dev::kVtSmem));

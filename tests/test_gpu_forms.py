@@ -1,5 +1,8 @@
 """The switches between the step's forms: which kernels a step runs, and what comes out."""
 import ctypes
+import os
+import subprocess
+import sys
 
 import numpy as np
 import pytest
@@ -68,3 +71,28 @@ def test_lists_asked_for_leave_the_fused_form(lib):
     _lanes(lib, 0, 4)
     lib.step()
     assert _tuning(lib)[0] == 0.0
+
+
+SMALL = """
+import ctypes, sys
+sys.path.insert(0, sys.argv[1])
+import numpy as np
+import helpers as H
+lib, t = H.b200(), np.zeros(7, np.float32)
+lib.raw.xpbd_b200_set_fused(1)
+H.scenes.Scenario(H.scenes.make_scene(50, 1), []).setup(lib)
+lib.step()
+lib.raw.xpbd_b200_tuning.argtypes = [ctypes.c_void_p]
+lib.raw.xpbd_b200_tuning(t.ctypes.data)
+lib.destroy()
+print(int(t[0]), int(t[4]))
+"""
+
+
+def test_fused_form_without_tiles():
+    """A scene too small for tiles, the first of its process, takes the fused launch too."""
+    tests = os.path.dirname(os.path.abspath(__file__))
+    env = dict(os.environ, PYTHONPATH=os.pathsep.join([H.ROOT, os.environ.get("PYTHONPATH", "")]))
+    r = subprocess.run([sys.executable, "-c", SMALL, tests], capture_output=True, text=True, timeout=300, env=env)
+    assert r.returncode == 0, r.stderr
+    assert r.stdout.split() == ["1", "1"]
