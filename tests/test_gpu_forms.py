@@ -96,3 +96,54 @@ def test_fused_form_without_tiles():
     r = subprocess.run([sys.executable, "-c", SMALL, tests], capture_output=True, text=True, timeout=300, env=env)
     assert r.returncode == 0, r.stderr
     assert r.stdout.split() == ["1", "1"]
+
+
+def _one_iteration(positions, scene, lanes, members=32):
+    """One substep of one volume iteration from ``positions``, the gather's lanes set before it."""
+    solver = H.b200()
+    H.scenes.Scenario(scene, [], iters=1, shape=False, max_members=members).setup(solver)
+    solver.set_constraints(distance=False, shape=False, angle=False, volume=True)
+    _lanes(solver, 0, lanes)
+    solver.step()
+    solver.reset()
+    solver.set_positions(positions)
+    solver.step()
+    tiles = solver.ints("gather_tiles")
+    _lanes(solver, 0, 0)
+    out = solver.positions()
+    solver.destroy()
+    return out, tiles
+
+
+POSES = {
+    "half pressed flat": lambda p: np.where(p[:, :1] > 0.0, p * [1.0, 1.0, 0.05], p),
+    "half pressed": lambda p: np.where(p[:, :1] > 0.0, p * [1.0, 1.0, 0.3], p),
+    "pressed": lambda p: p * [1.0, 1.0, 0.5],
+    "drawn out": lambda p: p * [3.0, 1.0, 1.0],
+}
+
+
+@pytest.mark.parametrize("pose", POSES)
+def test_large_records_leave_the_tile_form(pose):
+    """One tile, some of whose clusters are far from their volume: rounded to 23 bits of the
+    largest, the records of all would move the points by other amounts than the lists' floats do.
+    Taken from the lists, the moves (up to 0.03) differ by the order of a few FP32 operations, a
+    relative 2^-24, which turns one rounding in 25 of positions around 0.5; twice that is let pass."""
+    scene = H.scenes.make_scene(128, 3)
+    pos = POSES[pose](scene["pos"] * 1.01).astype(np.float32)
+    tile, (tiles, rows) = _one_iteration(pos, scene, 0)
+    lists, _ = _one_iteration(pos, scene, 4)
+    assert tiles == 1 and rows == 0
+    assert np.mean(tile != lists) < 0.08
+
+
+def test_small_records_take_the_tile_form():
+    """Swollen by 1 %: the tile form runs (its roundings show) and is off by at most 2^-27 of the
+    largest coordinate, which can turn the rounding of a position, one unit of 2^-23, either way."""
+    scene = H.scenes.make_scene(128, 3)
+    pos = (scene["pos"] * 1.01).astype(np.float32)
+    tile, (tiles, rows) = _one_iteration(pos, scene, 0)
+    lists, _ = _one_iteration(pos, scene, 4)
+    assert tiles == 1 and rows == 0
+    assert (tile != lists).any()
+    assert np.abs(tile.astype(np.float64) - lists).max() <= (2.0 ** -23 + 2.0 ** -27) * np.abs(pos).max()
