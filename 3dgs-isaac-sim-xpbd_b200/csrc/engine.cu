@@ -758,8 +758,10 @@ public:
 	// The gather's tiles of 128 rows.  Rows go along the curve, component by component, in
 	// equal tiles, so a tile depends on its component alone (an object's result is the same
 	// alone, packed with others or renumbered).  Rows without entries, rows of small
-	// components and of tiles that do not pay (k_tile_build) keep the list form, row by row.
-	int build_tiles(const std::vector<int>& off_h)
+	// components and of tiles that do not pay keep the list form, row by row.  Whether a tile's
+	// lists are long enough (kVtMinEntries) is known here; the rest k_tile_build finds out.
+	// by_length: all rows in length_order, which the lists take if no row is in a tile.
+	int build_tiles(const std::vector<int>& off_h, const std::vector<int>& by_length)
 	{
 		tiles.release();
 		std::vector<int> order(n), rank;
@@ -774,24 +776,24 @@ public:
 		}
 		std::vector<dev::VolTile> list;
 		std::vector<int> rows, active, plain;
+		std::vector<char> tiled(n, 0);
 		rows.reserve(n);
 		long long entries = 0;
 		for (int b = 0; b < n;) {
+			const int comp = comp_no[perm[order[b]]];
 			int e = b;
-			while (e < n && comp_no[perm[order[e]]] == comp_no[perm[order[b]]]) ++e;
+			while (e < n && comp_no[perm[order[e]]] == comp) ++e;
 			active.clear();
-			for (int k = b; k < e; ++k) {
-				const int r = order[k], len = off_h[r + 1] - off_h[r];
-				if (e - b >= dev::kVtMinComponent && len > 0) {
-					active.push_back(r);
-					entries += len;
-				}
-				else
-					plain.push_back(r);
-			}
+			if (e - b >= dev::kVtMinComponent)
+				for (int k = b; k < e; ++k)
+					if (off_h[order[k] + 1] > off_h[order[k]]) active.push_back(order[k]);
 			const long long count = (long long)active.size(), k = (count + dev::kVtRows - 1) / dev::kVtRows;
 			for (long long t = 0; t < k; ++t) {
 				const int a0 = (int)(count * t / k), a1 = (int)(count * (t + 1) / k), m = a1 - a0;
+				long long held = 0;
+				for (int a = a0; a < a1; ++a) held += off_h[active[a] + 1] - off_h[active[a]];
+				if (held < (long long)dev::kVtMinEntries * m) continue;
+				entries += held;
 				dev::VolTile v = {};
 				v.row0 = (int)rows.size();
 				v.nrows = m;
@@ -812,10 +814,16 @@ public:
 		// tiles that pay, then the rows of the others
 		std::vector<dev::VolTile> kept;
 		for (const auto& v : list)
-			if (v.cols) kept.push_back(v);
-			else plain.insert(plain.end(), rows.begin() + v.row0, rows.begin() + v.row0 + v.nrows);
-		std::sort(plain.begin(), plain.end());
-		length_order(plain, off_h);
+			if (v.cols) {
+				kept.push_back(v);
+				for (int k = 0; k < v.nrows; ++k) tiled[rows[v.row0 + k]] = 1;
+			}
+		if (kept.empty()) plain = by_length;
+		else {
+			for (int r = 0; r < n; ++r)
+				if (!tiled[r]) plain.push_back(r);
+			length_order(plain, off_h);
+		}
 		tiles.count = (int)kept.size();
 		tiles.list_count = (int)plain.size();
 		if (tiles.count)
@@ -877,6 +885,7 @@ public:
 		CK(cudaMemcpyAsync(vol_idx.p, vidx_i.data(), sizeof(int) * vidx_i.size(), cudaMemcpyHostToDevice, stream));
 		CK(cudaMemcpyAsync(rev_off.p, roff_i.data(), sizeof(int) * (n + 1), cudaMemcpyHostToDevice, stream));
 		CK(cudaMemcpyAsync(rev_idx.p, ridx_i.data(), sizeof(int) * ridx_i.size(), cudaMemcpyHostToDevice, stream));
+		std::vector<int> ord(n);   // rows in length_order
 		{
 			// copies of both lists with every row sorted along the curve of the component
 			// (caller index breaking ties), for the 4- and 8-lane kernels: the lanes of a cluster
@@ -914,18 +923,14 @@ public:
 				vol_pack.p, 1);
 			CK(cudaGetLastError());
 			CK(cudaMemcpyAsync(rev_idx_s.p, rs.data(), sizeof(int) * rs.size(), cudaMemcpyHostToDevice, stream));
-			{
-				std::vector<int> ord(n);
-				for (int r = 0; r < n; ++r) ord[r] = r;
-				length_order(ord, roff_i);
-				CK(gather_order.alloc(n));
-				CK(cudaMemcpyAsync(gather_order.p, ord.data(), sizeof(int) * n, cudaMemcpyHostToDevice, stream));
-				CK(cudaStreamSynchronize(stream));
-			}
+			for (int r = 0; r < n; ++r) ord[r] = r;
+			length_order(ord, roff_i);
+			CK(gather_order.alloc(n));
+			CK(cudaMemcpyAsync(gather_order.p, ord.data(), sizeof(int) * n, cudaMemcpyHostToDevice, stream));
 			CK(cudaStreamSynchronize(stream));
 			build_mark(5);
 		}
-		if (build_tiles(roff_i)) return -1;
+		if (build_tiles(roff_i, ord)) return -1;
 		build_mark(5);
 		vol_gs_order.release();
 		std::vector<int> order_i(clusters.gs_order.size());

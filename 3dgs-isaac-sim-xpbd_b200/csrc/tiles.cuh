@@ -91,8 +91,8 @@ constexpr int kVtHash = 8192;
 constexpr int kVtBuildSmem = (kVtCols + kVtGroups * (kVtCols / 32) * 16) * 4;
 
 // rank / row_of: position of a row along the curve and back (null: the same).  cols = 0 marks a
-// tile whose rows keep the list form: short lists (kVtMinEntries), more columns than kVtCols,
-// a list with a repeated or invalid entry, or masks that take more words than the lists.
+// tile whose rows keep the list form: more columns than kVtCols, a list with a repeated or
+// invalid entry, or masks that take more words than the lists.
 __global__ void __launch_bounds__(kVtThreads) k_tile_build(int n, VolTile* __restrict__ tiles,
 	const int* __restrict__ rows, const int* __restrict__ off, const int* __restrict__ idx,
 	const int* __restrict__ rank, const int* __restrict__ row_of, const float4* __restrict__ rest,
@@ -209,7 +209,7 @@ __global__ void __launch_bounds__(kVtThreads) k_tile_build(int n, VolTile* __res
 		s_groups[0] = s_pairs[0] = 0;
 		for (int g = 0; g < kVtGroups; ++g) { s_groups[g + 1] += s_groups[g]; s_pairs[g + 1] += s_pairs[g]; }
 		const int words = vt_pad(U) + vt_pad(s_groups[kVtGroups]) + 32 * s_pairs[kVtGroups];
-		if (!s_bad && words <= s_members && s_members >= kVtMinEntries * T.nrows) {
+		if (!s_bad && words <= s_members) {
 			s_base = atomicAdd(bump, (unsigned int)words);
 			if ((unsigned long long)s_base + words > pool_cap) s_bad = 1;
 		}
