@@ -1497,6 +1497,17 @@ public:
 			(!S.use_volume || (vol_lanes() == 4 && S.lanes_a == 0 && gather_lanes() == 4 && S.lanes_b == 0)) && !S.use_angle && n > 0;
 	}
 
+	// two rounds of clusters per warp (its 3x3 work on 16 lanes) where that still leaves every
+	// SM its 40 resident warps: 148 us a launch at 1M against 164 with one round; with four
+	// rounds 147, but 49 against 43 at 200,000 (a last wave of few blocks)
+	bool solve_two_rounds() const { return n >= 148 * 40 * 2 * dev::kSolveClusters; }
+
+	// whether forms 2 and 3 are kernels of their own: the automatic solve's two rounds
+	bool occ_forms() const
+	{
+		return S.use_volume && vol_lanes() == 4 && S.lanes_a == 0 && !vol_gs_on() && solve_two_rounds();
+	}
+
 	// the sorted lists unpacked, before a step that reads them
 	int ensure_sorted_members()
 	{
@@ -1512,10 +1523,7 @@ public:
 
 	void enqueue_volume_solve(const float4* pin, int read_lam, int occ)
 	{
-		// two rounds of clusters per warp (its 3x3 work on 16 lanes) where that still leaves every
-		// SM its 40 resident warps: 148 us a launch at 1M against 164 with one round; with four
-		// rounds 147, but 49 against 43 at 200,000 (a last wave of few blocks)
-		const bool many = n >= 148 * 40 * 2 * dev::kSolveClusters;
+		const bool many = solve_two_rounds();
 		const int rounds = many ? 2 : 1;
 		auto k = !many ? dev::k_volume_solve_warp<1, 5> : occ == 8 ? dev::k_volume_solve_warp<2, 8>
 			: occ == 6 ? dev::k_volume_solve_warp<2, 6> : dev::k_volume_solve_warp<2, 5>;
@@ -1784,7 +1792,7 @@ public:
 				form_kernels[0] = graph_kernels;
 				// the other forms; one that fails to capture is left out (the sequence carries on)
 				for (int f = 1; f < kForms; ++f) {
-					const bool want = (f == 1) ? (S.fused != 0 && fused_eligible()) : (S.fused == 2);
+					const bool want = (f == 1) ? (S.fused != 0 && fused_eligible()) : (S.fused == 2 && occ_forms());
 					if (want && capture(f, &graph_form[f], &form_kernels[f])) {
 						cudaGetLastError();
 						graph_form[f] = nullptr;

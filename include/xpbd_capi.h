@@ -215,7 +215,7 @@ XPBD_API void xpbd_b200_set_graph(int enabled);
  * substep as ONE cooperative launch with grid-wide barriers between its phases (form 1,
  * where the configuration allows it: no self-collision, object mode or Gauss-Seidel
  * forms); the sequence with its volume solve compiled for 6 or 8
- * resident blocks per SM (forms 2, 3).  Mode 0 (default) runs form 0, 1 runs form 1,
+ * resident blocks per SM (forms 2, 3; from 94,720 rows on, below which there is one).  Mode 0 (default) runs form 0, 1 runs form 1,
  * 2 lets the autotuner time every form on the first steps after each capture and keep
  * the fastest.  xpbd_b200_tuning fills out[7]: form in use, decided, mean trial ms of
  * forms 0 and 1, launches per step of the form in use, mean trial ms of forms 2 and 3. */

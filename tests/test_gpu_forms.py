@@ -147,3 +147,19 @@ def test_small_records_take_the_tile_form():
     assert tiles == 1 and rows == 0
     assert (tile != lists).any()
     assert np.abs(tile.astype(np.float64) - lists).max() <= (2.0 ** -23 + 2.0 ** -27) * np.abs(pos).max()
+
+
+def _settled(solver, n, mode):
+    """Positions after 24 substeps of a pinned scene in ``mode``, and the tuner's figures."""
+    scen = H.scenes.plain_scene_scenario(n, 2, pins=50)
+    scen.setup(solver)
+    _fused(solver, mode)
+    scen.advance(solver, 24)
+    return solver.positions(), _tuning(solver)
+
+
+def test_one_round_of_the_solve_has_no_other_forms(lib):
+    """Below two rounds the forms 2 and 3 would be form 0 again: they are not tried."""
+    _, t = _settled(lib, 2500, 2)
+    assert t[1] == 1.0 and t[0] in (0.0, 1.0) and t[2] > 0.0 and t[3] > 0.0
+    assert t[5] == 0.0 and t[6] == 0.0
