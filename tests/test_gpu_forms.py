@@ -163,3 +163,45 @@ def test_one_round_of_the_solve_has_no_other_forms(lib):
     _, t = _settled(lib, 2500, 2)
     assert t[1] == 1.0 and t[0] in (0.0, 1.0) and t[2] > 0.0 and t[3] > 0.0
     assert t[5] == 0.0 and t[6] == 0.0
+
+
+def test_forms_agree_above_two_rounds(lib):
+    """94,800 rows: two rounds of the solve, in all its forms, under the autotuner."""
+    out, t = _settled(lib, 94800, 2)
+    assert t[1] == 1.0 and (t[[2, 3, 5, 6]] > 0.0).all()
+    ref, _ = _settled(lib, 94800, 0)
+    assert H.max_err_over_diag(out, ref, H.scenes.bbox_diagonal(ref)) < H.TOL_1STEP
+
+
+def test_session_above_two_rounds_equals_alone():
+    """Alone, 40,000 rows take eight rows a warp in the distance kernel and one round of the
+    solve; in an arena of 100,000 both take the larger forms.  Same bits."""
+    serve = H.pkg.serve
+
+    def session(k, n):
+        s = serve.Session(k, 0.0, n, 99, 300 + k)
+        s.admit(H.B200_SO)
+        return s
+
+    sizes = (40000, 60000)
+    rows = sum(sizes)
+    arena = H.pkg.bridge.Arena(H.B200_SO, rows, rows * 12, rows * 66, rows * 68)
+    live = [session(k, n) for k, n in enumerate(sizes)]
+    for s in live:
+        s.slot = arena.admit(s.solver)
+        assert s.slot is not None
+        s.solver.close()
+    for _ in range(2):
+        arena.step(10, *serve._frame_arrays(live, 10))
+        arena.sync()
+        for s in live:
+            s.scen.k += 10
+    got = [arena.positions(s.slot, s.n) for s in live]
+    arena.close()
+    for k, n in enumerate(sizes):
+        alone = session(k, n)
+        for _ in range(2):
+            alone.enqueue_frame()
+        alone.solver.lib.xpbd_b200_sync()
+        np.testing.assert_array_equal(got[k], alone.solver.positions())
+        alone.close(keep_result=False)
