@@ -189,7 +189,7 @@ public:
 
 	// ---- device state ----
 	DBuf<float4> pos_curr, pos_next, pos_tmp, vel, pos_rest, shape_rest;
-	DBuf<float4> shape_q;    // per Gaussian: eigenvector frame of its last FP64 polar decomposition
+	DBuf<float4> shape_q;    // per Gaussian: the rotation of its last shape matching, a quaternion (zero: none)
 	// ChainMail: (arrival time, density) and the mask of changed Gaussians, each with the copy
 	// that a sweep writes; whether the last sweeps changed anything; seeds
 	DBuf<float2> cm_td, cm_td_next;

@@ -11,7 +11,7 @@ namespace dev {
 // commit, with a grid-wide barrier between phases.  Every phase runs the same
 // per-item code as its own kernel (the *_row / *_lane / tile functions, with plain
 // loads for the data the launch itself writes), so the result is that of the kernel
-// sequence bit for bit; what changes is one launch per substep instead of one per
+// sequence to FP32 rounding; what changes is one launch per substep instead of one per
 // phase.  Covers the default forms (Jacobi distance, 4-lane one-pass volume solve and
 // gather, shape matching, colliders, ground, press, contact shapes); self-collision,
 // object mode and the Gauss-Seidel forms keep the kernel sequence.

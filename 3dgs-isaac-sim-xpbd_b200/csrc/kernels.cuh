@@ -373,7 +373,7 @@ __device__ __forceinline__ bool distance_edge(float3 pi, float wi, float4 q4, fl
 	const float d0 = __fmul_rn(d2, inv);
 	const float d = __fmaf_rn(__fmaf_rn(-d0, d0, d2), __fmul_rn(0.5f, inv), d0);
 	const float denom = __fadd_rn(__fadd_rn(wi, __fmul_rn(q4.w, ims)), alpha_tilde);
-	// d2 below 1e-14 is a length below 1e-7 (and a NaN d from d2 = 0 or infinity)
+	// d2 below 1e-14 is a length below 1e-7 (d from d2 = 0 is NaN)
 	if (d2 < 1e-14f || denom < 1e-8f) return false;
 	const float dl = quotient(__fmaf_rn(-alpha_tilde, lambda, __fsub_rn(rest, d)), denom);
 	lambda = __fadd_rn(lambda, dl);

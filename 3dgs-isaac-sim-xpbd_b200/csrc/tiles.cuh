@@ -295,10 +295,6 @@ constexpr float kVtTop = 4194303.0f;       // 2^22 - 1: the largest value of a k
 constexpr float kVtMagic = 12582912.0f;    // 1.5 x 2^23: v + kVtMagic rounds v to an integer, whose
                                            // 2^22 + v are the low three bytes of the sum
 
-// The 32 rows of the two fragments come in pairs (r, r + 8) that lie side by side in a lane's
-// registers; pair k is rows 16 (k / 8) + k % 8 and 8 more.
-__host__ __device__ constexpr int vt_pair_row(int k, int second) { return 16 * (k / 8) + k % 8 + 8 * second; }
-
 // four columns' integers v + kVtMagic, byte by byte: the low, middle and high bytes of each
 struct VtWords { unsigned int high, mid, low; };
 __device__ __forceinline__ VtWords vt_bytes4(float v0, float v1, float v2, float v3)
@@ -311,8 +307,9 @@ __device__ __forceinline__ VtWords vt_bytes4(float v0, float v1, float v2, float
 	w.high = __byte_perm(__byte_perm(a, b, 0x0062), __byte_perm(c, d, 0x0062), 0x5410);
 	return w;
 }
-// where thread `quad`'s four columns go in the A-fragment order of m16n8k32; pair k of rows is
-// 8 bytes at vt_pair(k) from there
+// where thread `quad`'s four columns go in the A-fragment order of m16n8k32.  The 32 rows of the
+// two fragments come in pairs (r, r + 8) that lie side by side in a lane's registers; pair k,
+// rows 16 (k / 8) + k % 8 and 8 more, is 8 bytes at vt_pair(k) from there
 __device__ __forceinline__ unsigned char* vt_place(unsigned char* slab, int quad)
 {
 	return slab + (quad >> 3) * kVtChunk + (quad & 3) * 16 + ((quad >> 2) & 1) * 8;
@@ -324,13 +321,6 @@ __device__ __forceinline__ void vt_put(unsigned char* at, int k, unsigned int fi
 }
 
 __device__ __forceinline__ unsigned int vt_abs_bits(float v) { return __float_as_uint(v) & 0x7fffffffu; }
-
-// the four columns of this thread in the slab from column c0
-__device__ __forceinline__ int4 vt_columns(const VolTile& T, const unsigned int* __restrict__ words, int c0)
-{
-	const int c = c0 + 4 * (int)threadIdx.x;
-	return c < vt_pad(T.cols) ? *reinterpret_cast<const int4*>(words + c) : make_int4(-1, -1, -1, -1);
-}
 
 __device__ __forceinline__ void vt_copy16(void* to, const void* from)
 {

@@ -211,7 +211,7 @@ XPBD_API void xpbd_b200_set_volume_warp_mode(int mode);
 XPBD_API void xpbd_b200_set_volume_lanes(int solve_lanes, int gather_lanes);
 /* 1 (default): replay each step from a captured CUDA graph; 0: launch kernel by kernel. */
 XPBD_API void xpbd_b200_set_graph(int enabled);
-/* Step forms, all with the same results bit for bit: the kernel sequence (form 0); the
+/* Step forms, all with the same results to FP32 rounding: the kernel sequence (form 0); the
  * substep as ONE cooperative launch with grid-wide barriers between its phases (form 1,
  * where the configuration allows it: no self-collision, object mode or Gauss-Seidel
  * forms); the sequence with its volume solve compiled for 6 or 8
