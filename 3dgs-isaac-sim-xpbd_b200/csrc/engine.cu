@@ -191,10 +191,11 @@ public:
 	DBuf<float4> pos_curr, pos_next, pos_tmp, vel, pos_rest, shape_rest;
 	DBuf<float4> shape_q;    // per Gaussian: the rotation of its last shape matching, a quaternion (zero: none)
 	// ChainMail: (arrival time, density) and the mask of changed Gaussians, each with the copy
-	// that a sweep writes; whether the last sweeps changed anything; seeds
+	// that a sweep writes; whether the last sweeps changed anything, and which blocks of rows;
+	// each warp's near blocks; seeds
 	DBuf<float2> cm_td, cm_td_next;
 	DBuf<unsigned int> cm_mask, cm_mask_next;
-	DBuf<int> cm_changed, cm_seed_idx;
+	DBuf<int> cm_changed, cm_near, cm_seed_idx;
 	DBuf<float> cm_seed_delta, cm_time_out;
 	// object mode: rest offsets q (FP64, internal order), per-object rest centroid, sum q,
 	// count, previous centroid, fit parameters, centroid move, block partials, fit weights,
@@ -475,7 +476,7 @@ public:
 	{
 		pos_curr.release(); pos_next.release(); pos_tmp.release(); vel.release(); pos_rest.release();
 		shape_rest.release(); shape_q.release();
-		cm_td.release(); cm_td_next.release(); cm_mask.release(); cm_mask_next.release(); cm_changed.release();
+		cm_td.release(); cm_td_next.release(); cm_mask.release(); cm_mask_next.release(); cm_changed.release(); cm_near.release();
 		cm_seed_idx.release(); cm_seed_delta.release(); cm_time_out.release();
 		obj_q.release(); obj_shift.release(); obj_sumq.release(); obj_partial.release(); obj_c0.release();
 		obj_params.release(); obj_disp.release(); obj_w.release(); obj_boxes.release(); push_partial.release();
@@ -1070,6 +1071,7 @@ public:
 	// ------------------------------------------------------------------ ChainMail
 	// ensureChainmailGPU's time / density upload (forward.cu:10679-10698, 10826): every
 	// arrival time 1e9 (not reached), density = opacity.  Allocated on first use.
+	size_t cm_block_count() const { return ((size_t)n + (1 << dev::kCmBlock) - 1) >> dev::kCmBlock; }
 	int ensure_chainmail()
 	{
 		if (cm_td.p) return 0;
@@ -1077,7 +1079,10 @@ public:
 		std::vector<float2> td(n);
 		for (int i = 0; i < n; ++i) td[i] = make_float2(1e9f, dens[i]);
 		CK(cm_td_next.alloc(n)); CK(cm_mask.alloc((n + 31) / 32)); CK(cm_mask_next.alloc((n + 31) / 32));
-		CK(cm_time_out.alloc(n)); CK(cm_changed.alloc(4)); CK(cm_td.alloc(n));
+		CK(cm_near.alloc(dev::kCmNear * (((size_t)n + 31) / 32)));
+		CK(cm_time_out.alloc(n)); CK(cm_changed.alloc(4 * dev::kCmLine + 3 * cm_block_count())); CK(cm_td.alloc(n));
+		dev::k_cm_near<<<blocks_for(n, dev::kCmWarps * 32), dev::kCmWarps * 32, 0, stream>>>(n, off.p, nbr.p, cm_near.p);
+		CK(cudaGetLastError());
 		CK(cudaMemcpyAsync(cm_td.p, td.data(), sizeof(float2) * n, cudaMemcpyHostToDevice, stream));
 		CK(cudaMemsetAsync(cm_mask.p, 0, cm_mask.bytes(), stream));
 		return sync();
@@ -1115,9 +1120,11 @@ public:
 		float4* a = pos_curr.p;
 		float4* b = pos_tmp.p;
 		if (prop_iters) CK(cudaMemsetAsync(cm_changed.p, 0, cm_changed.bytes(), stream));
+		auto blocks = [&](int k) { return cm_changed.p + 4 * dev::kCmLine + (k % 3) * cm_block_count(); };
 		for (int it = 0; it < prop_iters; ++it) {
 			dev::k_cm_sweep<<<G, B, 0, stream>>>(n, it, S.cm_frontier ? 0 : 1, a, cm_td.p, b, cm_td_next.p, cm_mask.p,
-				cm_mask_next.p, cm_changed.p, off.p, nbr.p, ndist.p, nstiff.p, M, strength);
+				cm_mask_next.p, cm_changed.p, cm_near.p, blocks(it), blocks(it + 1), blocks(it + 2), off.p, nbr.p, ndist.p, nstiff.p, M,
+				strength);
 			++launches;
 			std::swap(a, b);
 			cm_td.swap(cm_td_next);

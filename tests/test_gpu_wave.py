@@ -1,0 +1,39 @@
+"""ChainMail waves that leave most of the scene alone: sweeps skip what they do not reach."""
+import numpy as np
+import pytest
+
+import helpers as H
+from test_gpu_rows import _hub_scene
+
+pytestmark = pytest.mark.gpu
+
+
+# blocks of 1,024 rows: one, a remainder of one row, several; rows whose edges lead to more blocks
+# than a warp lists (hubs of 12,000); waves that are under way, and long over, when the run ends
+@pytest.mark.parametrize("n,hubs,sweeps", [(1024, (), 5), (1025, (), 6), (6000, (), 4), (6000, (), 90),
+                                           (12000, (0, 7000), 3), (12000, (11999,), 40)])
+def test_waves_equal_dense_sweeps_and_oracle(n, hubs, sweeps):
+    """Two pushes, the second while the first wave is still a flag of changed rows.  Arrival times
+    are sums and minima of the same constants in the same order: equal."""
+    sc = _hub_scene(n, hubs)
+    sc["rest"] = (sc["rest"] * np.float32(1.01)).astype(np.float32)   # no edge at rest: see test_gpu_sweep.py
+    far = np.argsort(sc["pos"][:, 0])
+    out = []
+    for solver, frontier in ((H.b200(), 1), (H.b200(), 0), (H.oracle(), None)):
+        H.scenes.Scenario(sc, [], iters=1).setup(solver)
+        solver.step()
+        solver.reset()
+        if frontier is not None:
+            solver.lib.xpbd_b200_chainmail_set_frontier(frontier)
+        for k, seeds in enumerate((far[:3], far[-3:])):
+            solver.chainmail_seed(seeds.astype(np.int32), np.full((3, 3), 0.01 * (1 - 2 * k), np.float32))
+            solver.chainmail_run(**{**H.scenes.CHAINMAIL_DEFAULTS, "prop_iters": sweeps + k, "relax_iters": 0})
+        out.append((solver.positions(), solver.chainmail_times()))
+        if frontier is not None:
+            solver.lib.xpbd_b200_chainmail_set_frontier(1)
+        solver.destroy()
+    (p, t), (p_all, t_all), (q, u) = out
+    np.testing.assert_array_equal(t, t_all)
+    np.testing.assert_array_equal(p, p_all)
+    np.testing.assert_array_equal(t, u)
+    assert H.max_err_over_diag(p, q, H.scenes.bbox_diagonal(q)) < H.TOL_1STEP
