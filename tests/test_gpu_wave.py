@@ -27,7 +27,10 @@ def _scene(n, hubs):
                                            (12000, (0, 7000), 3), (12000, (11999,), 40)])
 def test_waves_equal_dense_sweeps_and_oracle(n, hubs, sweeps):
     """Two pushes, the second while the first wave is still a flag of changed rows.  Arrival times
-    are sums and minima of the same constants in the same order: equal."""
+    are sums and minima of the same constants in the same order: equal.  Positions equal those of
+    sweeps over every Gaussian, and after the first run the oracle's; its closing relax sweep leaves
+    edges at their rest length, where the second one's count of pulling edges is a matter of
+    rounding."""
     sc = _scene(n, hubs)
     far = np.argsort(sc["pos"][:, 0])
     out = []
@@ -37,15 +40,18 @@ def test_waves_equal_dense_sweeps_and_oracle(n, hubs, sweeps):
         solver.reset()
         if frontier is not None:
             solver.lib.xpbd_b200_chainmail_set_frontier(frontier)
+        runs = []
         for k, seeds in enumerate((far[:3], far[-3:])):
             solver.chainmail_seed(seeds.astype(np.int32), np.full((3, 3), 0.01 * (1 - 2 * k), np.float32))
             solver.chainmail_run(**{**H.scenes.CHAINMAIL_DEFAULTS, "prop_iters": sweeps + k, "relax_iters": 0})
-        out.append((solver.positions(), solver.chainmail_times()))
+            runs.append((solver.positions(), solver.chainmail_times()))
+        out.append(runs)
         if frontier is not None:
             solver.lib.xpbd_b200_chainmail_set_frontier(1)
         solver.destroy()
-    (p, t), (p_all, t_all), (q, u) = out
-    np.testing.assert_array_equal(t, t_all)
-    np.testing.assert_array_equal(p, p_all)
-    np.testing.assert_array_equal(t, u)
+    for (p, t), (p_all, t_all), (_, u) in zip(*out):
+        np.testing.assert_array_equal(p, p_all)
+        np.testing.assert_array_equal(t, t_all)
+        np.testing.assert_array_equal(t, u)
+    p, q = out[0][0][0], out[2][0][0]
     assert H.max_err_over_diag(p, q, H.scenes.bbox_diagonal(q)) < H.TOL_1STEP
