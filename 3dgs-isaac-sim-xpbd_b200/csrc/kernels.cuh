@@ -3124,7 +3124,9 @@ __global__ void __launch_bounds__(kBlock) k_jstats(int n, const float4* __restri
 // Bound by latency of the neighbours' records and of the two iterations: the matrices stay in
 // registers, a warp's neighbour indices come through shared memory (as in k_shape_match) and
 // two neighbours' records are in flight.  Two blocks per SM; three (80 registers) and four
-// (spills) are slower.  Measured (us per launch): 250,000 Gaussians 97 -> 54.
+// (spills) are slower.  Measured (us per launch): 250,000 Gaussians 97 -> 54, all deformed; of
+// 1,000,000 of which few have moved, with the projection that follows it, 145 -> 149 (152 where
+// every warp read its neighbours).
 // ---------------------------------------------------------------------------
 // Eigen-decomposition of a symmetric 3x3 matrix in FP64 by cyclic Jacobi sweeps over the
 // pivots (0,1), (0,2), (1,2) (symEig3Double's order and stop: off-diagonal mass below
@@ -3157,10 +3159,23 @@ __global__ void __launch_bounds__(kBlock, 2) k_deformed_shapes(int n, const floa
 	const int i = blockIdx.x * blockDim.x + threadIdx.x;
 	const int row0 = i & ~31;
 	if (row0 >= n) return;
+	// moved far enough for a deformation of its own?  A warp none of whose Gaussians did reads no
+	// neighbours
+	float3 x = make_float3(0.0f, 0.0f, 0.0f), x0 = x;
+	int e0 = 0, kn = 0;
+	if (i < n) {
+		x = f3(cur[i]);
+		x0 = f3(rest[i]);
+		e0 = off[i];
+		kn = off[i + 1] - e0;
+	}
+	const float dxv = x.x - x0.x, dyv = x.y - x0.y, dzv = x.z - x0.z;
+	const float diff = sqrtf(dxv * dxv + dyv * dyv + dzv * dzv);
+	const bool moved = diff > deform_eps && kn >= 3;
 	int* window = s_nbr[threadIdx.x >> 5];
 	const int begin = __ldg(off + row0), end = __ldg(off + min(row0 + 32, n));
 	const bool held = end - begin <= kShapeWindow;
-	if (held)
+	if (__any_sync(0xffffffffu, moved) && held)
 		for (int e = begin + (threadIdx.x & 31); e < end; e += 32) window[e - begin] = __ldg(nbr + e);
 	__syncwarp();
 	if (i >= n) return;
@@ -3168,14 +3183,10 @@ __global__ void __launch_bounds__(kBlock, 2) k_deformed_shapes(int n, const floa
 	const int o = perm ? perm[i] : i;   // output slot in the caller's order
 	const float3 s0 = make_float3(scales[3 * i], scales[3 * i + 1], scales[3 * i + 2]);
 	const float4 q0 = make_float4(rots[4 * i], rots[4 * i + 1], rots[4 * i + 2], rots[4 * i + 3]);
-	const float3 x = f3(cur[i]), x0 = f3(rest[i]);
-	const float dxv = x.x - x0.x, dyv = x.y - x0.y, dzv = x.z - x0.z;
-	const float diff = sqrtf(dxv * dxv + dyv * dyv + dzv * dzv);
-	const int e0 = off[i], kn = off[i + 1] - e0;
 	bool deformed = false;
 	M3 Sigma;
 	m3_zero(Sigma);
-	if (diff > deform_eps && kn >= 3) {
+	if (moved) {
 		M3 PPt, QPt;
 		m3_zero(PPt);
 		m3_zero(QPt);
