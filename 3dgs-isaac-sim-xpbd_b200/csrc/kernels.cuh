@@ -1957,7 +1957,7 @@ __device__ __forceinline__ void shape_row(int idx, int n, const StepParams* __re
 // A thread per Gaussian; a warp's edges are one run of the CSR array, so it brings their
 // neighbours to shared memory in a few coalesced loads first (one step of the dependent chain
 // less per trip; a run longer than the buffer is read in place).  Measured (us per launch,
-// the warm-started FP64 Jacobi -> this): 1,000,000 Gaussians 140 -> 100, 200,000 42 -> 27,
+// the warm-started FP64 Jacobi -> this): 1,000,000 Gaussians 140 -> 101, 200,000 42 -> 27,
 // 20,000 17 -> 12.7.  Three blocks per SM (80 registers): four spill, 98 and 32 us, five 110
 // and 36.
 constexpr int kShapeWindow = 448;
