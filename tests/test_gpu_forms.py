@@ -205,3 +205,26 @@ def test_session_above_two_rounds_equals_alone():
         alone.solver.lib.xpbd_b200_sync()
         np.testing.assert_array_equal(got[k], alone.solver.positions())
         alone.close(keep_result=False)
+
+
+@pytest.mark.parametrize("value", [np.nan, np.inf, 1e20, 50.0])
+def test_a_position_gone_astray_against_the_oracle(value):
+    """One Gaussian far off or not finite, in the middle of a tile: the others as the oracle has
+    them, finite where it has them finite."""
+    scene = H.scenes.make_scene(1500, 5)
+    pos = (scene["pos"] * [1.1, 0.95, 1.0]).astype(np.float32)
+    pos[700, 1] = value
+    out = []
+    for solver in (H.b200(), H.oracle()):
+        H.scenes.Scenario(scene, [], iters=1, shape=False).setup(solver)
+        solver.step()
+        solver.reset()
+        solver.set_positions(pos)
+        solver.step()
+        out.append(solver.positions())
+        solver.destroy()
+    got, ref = out
+    np.testing.assert_array_equal(np.isfinite(got), np.isfinite(ref))
+    near = np.isfinite(ref).all(1) & (np.abs(ref).max(1) < 10.0)
+    assert near.sum() >= 1480
+    assert H.max_err_over_diag(got[near], ref[near], H.scenes.bbox_diagonal(ref[near])) < H.TOL_1STEP
